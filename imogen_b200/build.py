@@ -16,9 +16,12 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 UNITS = ["imogen_b200.cu", "fluid_f32.cu", "fluid_f64.cu", "magnet_f32.cu", "magnet_f64.cu", "fluid_cluster.cu",
-         "matfile.cpp", "server.cpp"]
+         "seg_f32.cu", "seg_f64.cu", "win_f32.cu", "win_f64.cu", "matfile.cpp", "server.cpp"]
 # per-unit ptxas options: the batched cluster fluid kernels are compiled at -O1 (fluid_cluster.cu says why)
 UNIT_FLAGS = {"fluid_cluster.cu": ["-Xptxas", "-O1"]}
+# the window kernels are compiled without implicit FMA contraction: their FMAs are written out, so that every
+# instantiation (alone, batched, any block size) rounds alike and a batch equals its members alone bit for bit
+UNIT_FLAGS.update({u: ["-fmad=false"] for u in ("win_f32.cu", "win_f64.cu")})
 OUT = os.path.join(HERE, "libimogen_b200.so")
 HEADER = os.path.join(ROOT, "include", "imogen_b200.h")
 

@@ -251,6 +251,12 @@ __device__ __forceinline__ float rcp_approx(float x) {
     asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+// The same for an operand known not to be subnormal (subnormals count as 0): without the scaling around it.
+__device__ __forceinline__ float rcp_ftz(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 __device__ __forceinline__ float sqrt_approx(float x) {
     float r;
     asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));

@@ -25,6 +25,8 @@
 
 #include "../../include/imogen_b200.h"
 #include "cfl.cuh"
+#include "seg_fluid.cuh"
+#include "seg_magnet.cuh"
 #include "treadmill.cuh"
 
 using namespace img;
@@ -414,6 +416,15 @@ std::vector<PencilCfg> pencil_candidates(const Geom& g, int d, size_t elem) {
     return out;
 }
 
+// Block sizes that single-pencil CTAs along x are padded to: 64, 96, 128, 192, 256, 384, 512.
+int padded_block(int nt) {
+    for (int b = 64; b < 512; b *= 2) {
+        if (nt <= b) return b;
+        if (nt <= b + b / 2) return b + b / 2;
+    }
+    return nt <= 512 ? 512 : nt;
+}
+
 // Segment tilings of the fluid sweep (seg_fluid.cuh): C consecutive cells per thread (2, 3, 4 or 8; 2,
 // 3 or 4 in FP64; 2 or 4 with artificial viscosity), the whole pencil in one CTA of NT = Wb * S threads,
 // 64 <= NT <= 512, S = N / C threads per pencil.  Along x the S threads of a pencil are consecutive
@@ -477,13 +488,12 @@ std::vector<PencilCfg> seg_candidates(const Geom& g, int d, size_t elem, bool vi
     return out;
 }
 
-// Window tilings of the magnet chain and CT pass (seg_magnet.cuh): C = 2, 3, 4 or 8 consecutive cells per
-// thread with C dividing N, S = N / C threads per pencil, the whole pencil in one CTA of NT = Wb * S
-// threads (32 <= NT <= 512, a multiple of 32); along y and z Wb >= 4 pencils side by side (up to 64, or
-// to the CTA where each pencil is one thread's).  Along x, for a C where no such tiling exists, the
-// padded ones: S = ceil(N / C) segments (the last one ragged), NT = Wb * S rounded up to a multiple of
-// 32 with the threads past the segments idle, and for S above 256 (512) segments one pencil over a
-// cluster of CL = ceil(S / 256) <= 8 CTAs (ceil(S / 512) <= 4) of NT = ceil(S / CL) rounded up.
+// Window tilings of the magnet chain and CT pass (seg_magnet.cuh): C = 2, 3 (dividing N), 4 or 8 consecutive
+// cells per thread, S = ceil(N / C) threads per pencil (the last segment may be shorter), whole pencils in one
+// CTA of NT = Wb * S threads rounded up to a multiple of 32 (32 <= NT <= 512, the threads past the segments
+// idle); along y and z Wb >= 4 pencils side by side (2 where 4 do not fit; up to 64, or to the CTA where each
+// pencil is one thread's).  Along x, for S above 256 (512) segments, one pencil over a cluster of
+// CL = ceil(S / 256) <= 8 CTAs (ceil(S / 512) <= 4) of NT = ceil(S / CL) rounded up.
 std::vector<PencilCfg> win_candidates(const Geom& g, int d) {
     std::vector<PencilCfg> out;
     const int N = g.n[d];
@@ -499,27 +509,22 @@ std::vector<PencilCfg> win_candidates(const Geom& g, int d) {
         out.push_back(p);
     };
     for (int C : {2, 3, 4, 8}) {
-        const size_t before = out.size();
-        if (N % C == 0) {
-            const int S = N / C;
-            for (int Wb = d == 0 ? 1 : 4; Wb <= (d != 0 && S == 1 ? 512 : 64); Wb *= 2) {
-                const int NT = Wb * S;
-                if (NT > 512) break;
-                if (NT < 32 || NT % 32) continue;
-                if (Wb > 1 && (long long)Wb / 2 >= ncol) break;
-                add(Wb, S, 1, NT, C);
-            }
-        }
-        if (d != 0 || out.size() > before || C == 3) continue;
+        if (C == 3 && N % 3 != 0) continue;
         const int S = (N + C - 1) / C;
-        for (int Wb = 1; Wb * S <= 512; Wb *= 2) {
-            if (Wb > 1 && (long long)Wb / 2 >= ncol) break;
-            add(Wb, S, 1, std::max(32, (Wb * S + 31) / 32 * 32), C);
+        for (int Wb = d == 0 ? 1 : (4 * S <= 512 ? 4 : 2); Wb <= (d != 0 && S == 1 ? 512 : 64); Wb *= 2) {
+            const int NT = std::max(32, (Wb * S + 31) / 32 * 32);
+            if (NT > 512) break;
+            if (Wb > 1 && (long long)Wb / 2 >= ncol && Wb * S > 32) break;
+            add(Wb, S, 1, NT, C);
+            if (d == 0 && Wb == 1 && S >= 64 && padded_block(NT) != NT) add(1, S, 1, padded_block(NT), C);
         }
+        if (d != 0 || C == 3) continue;
         for (int cap : {256, 512}) {
             const int CL = (S + cap - 1) / cap;
             if (CL < 2 || CL > (cap == 256 ? 8 : 4)) continue;
-            add(1, S, CL, ((S + CL - 1) / CL + 31) / 32 * 32, C);
+            const int NT = ((S + CL - 1) / CL + 31) / 32 * 32;
+            add(1, S, CL, NT, C);
+            if (padded_block(NT) != NT) add(1, S, CL, padded_block(NT), C);
         }
     }
     return out;
@@ -542,11 +547,44 @@ const PencilCfg* default_segments(const std::vector<PencilCfg>& c, int d) {
     return best;
 }
 
+// Default window tiling of direction d among candidates c, with C = `want` cells per thread, or a
+// whole pencil in each thread where it has that few cells.  CTAs of about 256 threads (two or more share an
+// SM, so that one's loads and barriers hide behind another's arithmetic), smaller ones down to 64 while the
+// grid has fewer CTAs than two per SM (pencils of one thread exchange nothing and keep 256); along y and z rows
+// of at least 32 bytes (a memory sector) where that fits; few idle threads.  A long pencil along x that has
+// a CTA of its own takes a padded block size (padded_block), so that pencils of similar length share a
+// launch shape when they are batched.  nullptr: none.
+const PencilCfg* default_windows(const std::vector<PencilCfg>& c, const Geom& g, int d, size_t elem, int want) {
+    const int N = g.n[d];
+    const long long ncol = g.ncell / N;
+    const PencilCfg* best = nullptr;
+    double best_cost = 0;
+    for (const PencilCfg& p : c) {
+        if (p.seg != (N <= want ? N : want)) continue;
+        const long long ctas = (ncol + p.Wb - 1) / p.Wb * p.CL;
+        double cost = std::fabs(std::log2(p.NT / 256.0));
+        if (p.G > 1) {
+            if (p.NT < 256 && ctas < 4 * 148) cost *= 0.25;                       // small grids: spread out
+            if (ctas < 2 * 148) cost += 0.5 * std::log2(2.0 * 148 / ctas);
+        }
+        const double idle = 1.0 - (double)p.Wb * p.G / ((double)p.NT * p.CL);
+        if (d == 0 && p.Wb == 1 && p.G >= 64) cost = cost * 0.25 + 0.5 * idle + (padded_block(p.NT) == p.NT ? 0.0 : 1.0);
+        else cost += 2.0 * idle;
+        if (d != 0 && p.G > 1 && p.Wb * elem < 32) cost += 1.5 * std::log2(32.0 / (p.Wb * elem));
+        if (p.CL > 1) cost += 2.0 + 0.1 * p.CL;
+        if (!best || cost < best_cost) {
+            best = &p;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
 // Default magnet tiling: the window kernels where a default window tiling exists, else the tile
 // kernels' default.
-PencilCfg choose_window(const Geom& g, int d, const PencilCfg& tile) {
+PencilCfg choose_window(const Geom& g, int d, size_t elem, const PencilCfg& tile) {
     std::vector<PencilCfg> c = win_candidates(g, d);
-    const PencilCfg* best = default_segments(c, d);
+    const PencilCfg* best = default_windows(c, g, d, elem, 4);
     return best ? *best : tile;
 }
 
@@ -837,7 +875,18 @@ void fill_mag_args(img_ctx* ctx, int X, int I1, int I2, MagArgs& a) {
         a.actI_mom[q] = active_lin(c, ctx->g.ndims, CLS_MOM, I);
         a.actI_mag[q] = active_lin(c, ctx->g.ndims, CLS_MAG, I);
         a.init_mag[q] = ctx->init_mag[I - 1][d];
+        a.w_BI[q] = ctx->q[Q_BX + e];
+        a.inv_dI[q] = 1.0 / c.dgrid[e];
+        a.nI[q] = ctx->g.n[e];
+        a.sI[q] = (int)ctx->g.s[e];   // grids have fewer than 2^31 cells
+        a.first[q] = e == a.sg.d1;
     }
+    a.w_rho = ctx->q[Q_RHO];
+    a.w_pX = ctx->q[Q_PX + d];
+    a.w_BX = ctx->q[Q_BX + d];
+    a.w_CBX = ctx->q[Q_CBX + d];
+    a.w_CB2 = ctx->q[Q_CBX + I2 - 1];
+    a.inv_dx = 1.0 / c.dgrid[d];
     a.fade = ctx->fade_dev;
     a.fade_f = c.bc_infinity;
     a.bc_inf = c.bc_infinity;
@@ -860,7 +909,9 @@ int launch_magnet(img_ctx* ctx, int X, int I1, int I2) {
     a.sg = sweep_geom(ctx, d, pcf);
     MagArgs ac = a;
     ac.sg = sweep_geom(ctx, d, pcc);
-    PencilLaunch L = pencil_launch<T>(ctx, pcf, d, pcf.seg ? 0 : mag_smem_bytes<T>(pcf.G * pcf.cpt, pcf.Wb, pcf.nqc),
+    PencilLaunch L = pencil_launch<T>(ctx, pcf, d,
+                                      pcf.seg ? chain_win_smem_bytes<T>(pcf.NT, pcf.seg)
+                                              : mag_smem_bytes<T>(pcf.G * pcf.cpt, pcf.Wb, pcf.nqc),
                                       pcf.seg ? 1 : 2 / pcf.nqc, fade_on(ctx->cfg, d, CLS_MAG, CLS_MAG));
     PencilLaunch Lc = pencil_launch<T>(ctx, pcc, d, pcc.seg ? 0 : ctcell_smem_bytes<T>(pcc.G * pcc.cpt, pcc.Wb), 1,
                                        fade_on(ctx->cfg, d, CLS_MAG, CLS_MAG));
@@ -960,6 +1011,7 @@ int set_kernel_attributes(img_ctx* ctx) {
                 CK(chain_attributes<T>(cpt, optin));
             }
             CK(fluid_seg_attributes<T>(optin));
+            CK(chain_win_attributes<T>(optin));
             CK(cudaFuncSetAttribute(treadmill_detect_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kPencilSmemLimit));
             CK(cudaFuncSetAttribute(treadmill_shift_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1389,7 +1441,7 @@ int img_create(img_ctx** out, const img_config* cfg) {
             } else {
                 ctx->pcfg_mtile[kind - 1][d] = ctx->pcfg[kind][d];
                 if (tile_only) continue;
-                ctx->pcfg[kind][d] = choose_window(g, d, ctx->pcfg_mtile[kind - 1][d]);
+                ctx->pcfg[kind][d] = choose_window(g, d, ctx->elem, ctx->pcfg_mtile[kind - 1][d]);
             }
             if (kind == 0 && cfg->viscosity_type != IMG_VISC_NONE && g.n[d] >= 3) {
                 bool ok = false;

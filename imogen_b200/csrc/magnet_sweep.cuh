@@ -38,6 +38,13 @@ struct MagArgs {
     double bc_inf;
     const EdgeTable* edges;
     int init_mag[2];           // first assignment of velGrid/store.fluxR/wMag/flux of (I, X)
+    // what the window kernels read instead of deriving it in every thread: the arrays by role, the
+    // reciprocal spacings, and per component the extent and stride along dim I and whether I is the
+    // pencils' first transverse dimension (g.d1)
+    void *w_rho, *w_pX, *w_BX, *w_CBX, *w_CB2;
+    void* w_BI[2];
+    double inv_dx, inv_dI[2];
+    int nI[2], sI[2], first[2];
 };
 
 // ---- transverse (non-pencil) shifts used by the pointwise passes ----------------------------------

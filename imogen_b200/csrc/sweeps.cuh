@@ -2,9 +2,8 @@
 // kernel family and precision, built in parallel) and called by the host code.
 #pragma once
 
+#include "fluid_sweep.cuh"
 #include "magnet_sweep.cuh"
-#include "seg_fluid.cuh"
-#include "seg_magnet.cuh"
 
 namespace img {
 
@@ -29,6 +28,15 @@ struct PencilLaunch {
 template <typename T> cudaError_t launch_fluid_sweep(const FluidArgs& a, const PencilLaunch& L, bool mhd);
 template <typename T> cudaError_t launch_mag_chain(const MagArgs& a, const PencilLaunch& L);
 template <typename T> cudaError_t launch_mag_ctcell(const MagArgs& a, const PencilLaunch& L);
+// The segment fluid and window magnet kernels (L.seg cells per thread), in units of their own; the
+// entry points above hand the launches with L.seg on to them.
+template <typename T> cudaError_t launch_fluid_seg(const FluidArgs& a, const PencilLaunch& L, bool mhd);
+template <typename T>
+cudaError_t launch_fluid_seg_batch(const FluidArgs* args, const BlockMap* map, const PencilLaunch& L, bool mhd);
+template <typename T> cudaError_t launch_mag_chain_win(const MagArgs& a, const PencilLaunch& L);
+template <typename T> cudaError_t launch_mag_ct_win(const MagArgs& a, const PencilLaunch& L);
+template <typename T> cudaError_t launch_mag_chain_win_batch(const MagArgs* args, const BlockMap* map, const PencilLaunch& L);
+template <typename T> cudaError_t launch_mag_ct_win_batch(const MagArgs* args, const BlockMap* map, const PencilLaunch& L);
 // Batched forms: one launch over the CTAs of many grids; `args` and `map` are device arrays (one
 // argument block per member, one BlockMap per CTA of the launch, L.grid_x CTAs).
 template <typename T>
@@ -46,6 +54,7 @@ cudaError_t launch_mag_ctcell_batch(const MagArgs* args, const BlockMap* map, co
 // batched, use up to `optin` bytes of shared memory per block (the device's opt-in maximum).
 template <typename T> cudaError_t fluid_attributes(int cpt, int optin);
 template <typename T> cudaError_t chain_attributes(int cpt, int optin);
+template <typename T> cudaError_t chain_win_attributes(int optin);   // the window chain kernels
 // Clusters of the MHD fluid kernel that can be co-resident for launch shape L (0: not schedulable).
 template <typename T> cudaError_t fluid_max_clusters(const PencilLaunch& L, int* n);
 // Shared-memory attributes of the segment fluid kernels (2, 3, 4 and 8 cells per thread; 2, 3 and 4 in

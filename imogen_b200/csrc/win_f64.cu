@@ -1,0 +1,10 @@
+// Window magnet kernels in double: the launch entry points of sweeps.cuh for this precision.
+#include "seg_impl.cuh"
+
+namespace img {
+template cudaError_t launch_mag_chain_win<double>(const MagArgs&, const PencilLaunch&);
+template cudaError_t launch_mag_ct_win<double>(const MagArgs&, const PencilLaunch&);
+template cudaError_t launch_mag_chain_win_batch<double>(const MagArgs*, const BlockMap*, const PencilLaunch&);
+template cudaError_t launch_mag_ct_win_batch<double>(const MagArgs*, const BlockMap*, const PencilLaunch&);
+template cudaError_t chain_win_attributes<double>(int);
+}  // namespace img
