@@ -1,7 +1,7 @@
 """Build the in-tree CUDA library libimogen_b200.so for sm_100a (nvcc, no JIT cache).
 
-The kernels are split over several translation units (host code; fluid and magnet sweeps per
-precision; the MAT-file slice reader/writer, host C++ linked with zlib) that compile in parallel and
+The kernels are split over several translation units (host code; fluid and magnet pencil-tile sweeps, segment
+fluid and window magnet kernels per precision; the MAT-file slice reader/writer, host C++ linked with zlib) that compile in parallel and
 link into one shared library with the CUDA runtime linked statically."""
 from __future__ import annotations
 
@@ -19,9 +19,9 @@ UNITS = ["imogen_b200.cu", "fluid_f32.cu", "fluid_f64.cu", "magnet_f32.cu", "mag
          "seg_f32.cu", "seg_f64.cu", "win_f32.cu", "win_f64.cu", "matfile.cpp", "server.cpp"]
 # per-unit ptxas options: the batched cluster fluid kernels are compiled at -O1 (fluid_cluster.cu says why)
 UNIT_FLAGS = {"fluid_cluster.cu": ["-Xptxas", "-O1"]}
-# the window kernels are compiled without implicit FMA contraction: their FMAs are written out, so that every
+# the segment and window kernels are compiled without implicit FMA contraction: their FMAs are written out, so that every
 # instantiation (alone, batched, any block size) rounds alike and a batch equals its members alone bit for bit
-UNIT_FLAGS.update({u: ["-fmad=false"] for u in ("win_f32.cu", "win_f64.cu")})
+UNIT_FLAGS.update({u: ["-fmad=false"] for u in ("seg_f32.cu", "seg_f64.cu", "win_f32.cu", "win_f64.cu")})
 OUT = os.path.join(HERE, "libimogen_b200.so")
 HEADER = os.path.join(ROOT, "include", "imogen_b200.h")
 

@@ -45,6 +45,8 @@ struct FluidArgs {
     double vc1, vc2, vk1, vk2, vc1sq;
     double minmass_out;    // the final max(rho, MINMASS) (relaxingFluid.m:71); -inf when a point-fade pass
                            // follows the sweep (it fades, clamps and fades again, as the two sets do)
+    double inv_dx;         // 1 / dx (segment kernels)
+    int round_cells;       // segment kernels: each cell that ends a group of so many rounds its half step's change (seg_predict); 0: none
 };
 constexpr int VISC_NONE = 0;
 constexpr int VISC_NR = 1;    // Neumann-Richtmyer (ArtificialViscosity.m:73-77)
@@ -97,7 +99,7 @@ __device__ __forceinline__ void wflux(int d, const T u[5], const T bb[3], T pres
         for (int v = 0; v < 5; ++v) w[v] = w[v] * ic;
     } else {   // plain FP64: wFluidFlux.m's terms, its divisions by rho and c_f as products with one
                // reciprocal of each (a rounding-level difference)
-        const T ir = T(1) / u[0], ic = T(1) / cf;
+        const T ir = recip(u[0]), ic = recip(cf);
         T velocity = pX * ir;
         w[0] = pX * ic;
         T we = velocity * (u[4] + press) - bX * (bb[0] * u[1] + bb[1] * u[2] + bb[2] * u[3]) * ir;
@@ -121,7 +123,7 @@ __device__ __forceinline__ T press_speed(double G, int d, const T u[5], double m
     } else {
         PressOut o = pressure_totsnd(G, u[0], u[1], u[2], u[3], u[4], msq);
         p = o.p + 0.0;   // + viscosity.solve ('empty' -> 0)
-        return fabs(pX * (1.0 / u[0])) + o.cs;
+        return fabs(pX * recip(u[0])) + o.cs;
     }
 }
 

@@ -25,6 +25,7 @@
 
 #include "../../include/imogen_b200.h"
 #include "cfl.cuh"
+#include "launch.cuh"
 #include "seg_fluid.cuh"
 #include "seg_magnet.cuh"
 #include "treadmill.cuh"
@@ -48,6 +49,7 @@ struct PencilCfg {
     int Wb = 1, G = 32, CL = 1, NT = 32, cpt = 2;
     int nqc = 1;   // magnet chain: transverse components per CTA
     int seg = 0;   // fluid sweep: segment kernel with seg = cpt consecutive cells per thread (G = N / cpt)
+    bool picked = false;   // by the autotuner or img_set_tiling, not a default
 };
 
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -134,7 +136,7 @@ inline bool pencil_kind(int kind) { return kind == OP_FLUID || kind == OP_CHAIN 
 struct OpRec {
     int kind;
     int elem;                 // 4 (mixed) or 8 (FP64)
-    bool mhd;                 // fluid: MHD variant
+    int mhd;                  // fluid: MHD variant (0: none; segment kernels: the form of the fluxes)
     PencilLaunch L;           // pencil kernels: this member's launch shape
     unsigned blocks;          // pointwise kernels: this member's block count
     FluidArgs fa;
@@ -426,63 +428,57 @@ int padded_block(int nt) {
 }
 
 // Segment tilings of the fluid sweep (seg_fluid.cuh): C consecutive cells per thread (2, 3, 4 or 8; 2,
-// 3 or 4 in FP64; 2 or 4 with artificial viscosity), the whole pencil in one CTA of NT = Wb * S threads,
-// 64 <= NT <= 512, S = N / C threads per pencil.  Along x the S threads of a pencil are consecutive
-// lanes: S is a power of two up to 32 or a multiple of 32.  Along y and z Wb >= 4 pencils (a power of
-// two) sit side by side, at most 32 of them unless each pencil is one thread's (S = 1).  Along x, for a
-// C (2, 4 or 8) with none of these and S = ceil(N / C) >= 64 segments, the cluster forms (seg_fluid.cuh's
-// CLU; no artificial viscosity): one pencil per CTA of NT = S rounded up to a multiple of 32 threads,
-// or over a cluster of CL = ceil(S / 256) <= 8 CTAs (ceil(S / 512) <= 4) of NT = ceil(S / CL) rounded
-// up; where C does not divide N the last segment is ragged (launch_fluid takes these for const ends
-// only).
-bool seg_cluster_form(const PencilCfg& p, int N) {
-    return p.seg && (p.CL > 1 || N % p.seg != 0 || p.NT != p.Wb * p.G);
+// 3 or 4 in FP64), S = ceil(N / C) threads per pencil (the last segment may be shorter), whole pencils in one
+// CTA of NT = Wb * S threads rounded up to a multiple of 32, 64 <= NT <= 512.  Along y and z Wb >= 4 pencils
+// (a power of two; 2 where 4 do not fit the CTA or its shared memory) sit side by side, at most 32 of them unless each pencil is one
+// thread's (S = 1).  Along x a pencil of more than 256 (512) segments may span a cluster of
+// CL = ceil(S / 256) <= 8 CTAs (ceil(S / 512) <= 4) of NT = ceil(S / CL) rounded up (seg_fluid.cuh's CLU).
+// With artificial viscosity every segment is whole, CTAs have no idle threads, C is 2 or 4, and along x S is
+// a power of two up to 32 or a multiple of 32.
+bool seg_cluster_form(const PencilCfg& p) { return p.seg && p.CL > 1; }
+
+size_t seg_smem(size_t elem, int NT, int Wb, bool visc, bool fade) {
+    return elem == 8 ? seg_fluid_smem_bytes<double>(NT, Wb, visc, fade) : seg_fluid_smem_bytes<float>(NT, Wb, visc, fade);
 }
 
 std::vector<PencilCfg> seg_candidates(const Geom& g, int d, size_t elem, bool visc = false) {
     std::vector<PencilCfg> out;
     const int N = g.n[d];
     const long long ncol = g.ncell / N;
+    auto add = [&](int Wb, int S, int CL, int NT, int C) {
+        if (seg_smem(elem, NT, Wb, visc, !visc && CL == 1) > kPencilSmemLimit) return;
+        PencilCfg p;
+        p.Wb = Wb;
+        p.G = S;
+        p.CL = CL;
+        p.NT = NT;
+        p.cpt = C;
+        p.seg = C;
+        out.push_back(p);
+    };
     for (int C : {2, 3, 4, 8}) {
         if ((elem == 8 && C == 8) || (visc && (C == 8 || C == 3))) continue;
-        const size_t before = out.size();
-        auto add_cluster = [&](int S, int CL, int NT) {
-            const size_t smem = elem == 8 ? seg_fluid_smem_bytes<double>(NT) : seg_fluid_smem_bytes<float>(NT);
-            if (smem > kPencilSmemLimit) return;
-            PencilCfg p;
-            p.Wb = 1;
-            p.G = S;
-            p.CL = CL;
-            p.NT = NT;
-            p.cpt = C;
-            p.seg = C;
-            out.push_back(p);
-        };
-        const int Se = N / C;
-        const bool exact = N % C == 0 && (d != 0 || Se % 32 == 0 || (Se <= 32 && 32 % Se == 0));
-        for (int Wb = d == 0 ? 1 : 4; exact && Wb <= (d != 0 && Se == 1 ? 512 : 32); Wb *= 2) {
-            const int NT = Wb * Se;
-            if (NT > 512) break;
-            if (NT < 64 || NT % 32) continue;
-            if (Wb > 1 && (long long)Wb / 2 >= ncol) break;   // more pencil slots than pencils
-            const size_t smem = elem == 8 ? seg_fluid_smem_bytes<double>(NT, visc) : seg_fluid_smem_bytes<float>(NT, visc);
-            if (smem > kPencilSmemLimit) continue;
-            PencilCfg p;
-            p.Wb = Wb;
-            p.G = Se;
-            p.CL = 1;
-            p.NT = NT;
-            p.cpt = C;
-            p.seg = C;
-            out.push_back(p);
-        }
-        if (d != 0 || visc || C == 3 || out.size() > before) continue;
+        if (C == 3 && N % 3 != 0) continue;
         const int S = (N + C - 1) / C;
-        if (S < 64) continue;
-        if (S <= 512) add_cluster(S, 1, (S + 31) / 32 * 32);
+        const bool exact = N % C == 0 && (d != 0 || S % 32 == 0 || (S <= 32 && 32 % S == 0));
+        if (visc && !exact) continue;
+        const int Wb0 = d == 0 ? 1 : (4 * S <= 512 && seg_smem(elem, 4 * S, 4, visc, !visc) <= kPencilSmemLimit ? 4 : 2);
+        for (int Wb = Wb0; Wb <= (d != 0 && S == 1 ? 512 : 32); Wb *= 2) {
+            const int NT = (Wb * S + 31) / 32 * 32;
+            if (NT > 512) break;
+            if (NT < 64 || (visc && (NT != Wb * S || Wb < Wb0))) continue;
+            if (Wb > 1 && (long long)Wb / 2 >= ncol && Wb * S > 64) break;   // more pencil slots than pencils
+            if (Wb == 2 && d != 0 && visc) continue;
+            add(Wb, S, 1, NT, C);
+            if (!visc && d == 0 && Wb == 1 && S >= 64 && padded_block(NT) != NT) add(1, S, 1, padded_block(NT), C);
+        }
+        if (d != 0 || visc || C == 3 || S < 64) continue;
         for (int cap : {256, 512}) {
             const int CL = (S + cap - 1) / cap;
-            if (CL >= 2 && CL <= (cap == 256 ? 8 : 4)) add_cluster(S, CL, ((S + CL - 1) / CL + 31) / 32 * 32);
+            if (CL < 2 || CL > (cap == 256 ? 8 : 4)) continue;
+            const int NT = ((S + CL - 1) / CL + 31) / 32 * 32;
+            add(1, S, CL, NT, C);
+            if (padded_block(NT) != NT) add(1, S, CL, padded_block(NT), C);
         }
     }
     return out;
@@ -530,43 +526,20 @@ std::vector<PencilCfg> win_candidates(const Geom& g, int d) {
     return out;
 }
 
-// Default segment or window tiling among candidates c: 4 cells per thread (along y and z at least 8
-// pencils side by side), else whole pencils of one thread each (pencils of 2 to 8 cells across y or z);
-// the CTA nearest 256 threads.  nullptr: none of these.
-const PencilCfg* default_segments(const std::vector<PencilCfg>& c, int d) {
-    const PencilCfg* best = nullptr;
-    for (const PencilCfg& p : c) {
-        if (p.seg != 4 || (d != 0 && p.Wb < 8)) continue;
-        if (!best || std::abs(p.NT - 256) < std::abs(best->NT - 256)) best = &p;
-    }
-    if (best || d == 0) return best;
-    for (const PencilCfg& p : c) {
-        if (p.G != 1) continue;
-        if (!best || std::abs(p.NT - 256) < std::abs(best->NT - 256)) best = &p;
-    }
-    return best;
-}
-
-// Default window tiling of direction d among candidates c, with C = `want` cells per thread, or a
-// whole pencil in each thread where it has that few cells.  CTAs of about 256 threads (two or more share an
-// SM, so that one's loads and barriers hide behind another's arithmetic), smaller ones down to 64 while the
-// grid has fewer CTAs than two per SM (pencils of one thread exchange nothing and keep 256); along y and z rows
-// of at least 32 bytes (a memory sector) where that fits; few idle threads.  A long pencil along x that has
-// a CTA of its own takes a padded block size (padded_block), so that pencils of similar length share a
-// launch shape when they are batched.  nullptr: none.
-const PencilCfg* default_windows(const std::vector<PencilCfg>& c, const Geom& g, int d, size_t elem, int want) {
+// Default segment or window tiling of direction d among candidates c, with C = `want` cells per thread, or a
+// whole pencil in each thread where it has up to 4.  `threads`: the CTA size that measured best; `big` weighs
+// larger ones.  Along y and z rows of at least 32 bytes (a memory sector) where that fits; few idle threads.  A
+// long pencil along x that has a CTA of its own takes a padded block size (padded_block), so that pencils of
+// similar length share a launch shape when they are batched.  nullptr: none.
+const PencilCfg* default_segments(const std::vector<PencilCfg>& c, const Geom& g, int d, size_t elem, int want, int threads,
+                                  double big) {
     const int N = g.n[d];
-    const long long ncol = g.ncell / N;
     const PencilCfg* best = nullptr;
     double best_cost = 0;
     for (const PencilCfg& p : c) {
-        if (p.seg != (N <= want ? N : want)) continue;
-        const long long ctas = (ncol + p.Wb - 1) / p.Wb * p.CL;
-        double cost = std::fabs(std::log2(p.NT / 256.0));
-        if (p.G > 1) {
-            if (p.NT < 256 && ctas < 4 * 148) cost *= 0.25;                       // small grids: spread out
-            if (ctas < 2 * 148) cost += 0.5 * std::log2(2.0 * 148 / ctas);
-        }
+        if (p.seg != (N <= 4 ? N : want)) continue;
+        double cost = std::log2(p.NT / (double)(p.G == 1 ? 256 : threads));
+        cost = cost > 0 ? big * cost : -cost;
         const double idle = 1.0 - (double)p.Wb * p.G / ((double)p.NT * p.CL);
         if (d == 0 && p.Wb == 1 && p.G >= 64) cost = cost * 0.25 + 0.5 * idle + (padded_block(p.NT) == p.NT ? 0.0 : 1.0);
         else cost += 2.0 * idle;
@@ -580,21 +553,39 @@ const PencilCfg* default_windows(const std::vector<PencilCfg>& c, const Geom& g,
     return best;
 }
 
-// Default magnet tiling: the window kernels where a default window tiling exists, else the tile
-// kernels' default.
+// Grids whose threads of 4 cells would not fill the chip (under 148 x 256 of them): there each thread's own chain
+// of work is what takes the time, and 2 cells a thread in CTAs of 128 make the faster fluid sweeps (one iteration: 64^2
+// mixed 53 -> 45 us, 64^2 FP64 89 -> 75 us, 24^3 mixed 78 -> 68 us; 200^2 60 -> 57 us; 512^2 is past the line: x fluid
+// sweep 7.5 us with 4 cells, 9.2 us with 2).
+bool small_grid(const Geom& g) { return g.ncell < 4 * 148 * 256; }
+
+// Default magnet tiling: the window kernels where a default window tiling exists, else the tile kernels'
+// default.  4 cells a thread and CTAs of 256 threads (512 share an SM by two as well: rows of 32 bytes come
+// first; 256^3 mixed, y: 8 pencils in 512 threads 355 us, 4 in 256 threads 476 us).
 PencilCfg choose_window(const Geom& g, int d, size_t elem, const PencilCfg& tile) {
     std::vector<PencilCfg> c = win_candidates(g, d);
-    const PencilCfg* best = default_windows(c, g, d, elem, 4);
+    const PencilCfg* best = default_segments(c, g, d, elem, 4, small_grid(g) ? 128 : 256, 1.0);
     return best ? *best : tile;
 }
 
-// Default fluid tiling: in the mixed form the segment kernel where a default segment tiling exists
-// (default_segments); in FP64, and where none exists, the tile kernels' default (the FP64 segment kernel
-// needs more registers than it has; the autotuner may still pick it).
+// Default fluid tiling: the segment kernel where a default segment tiling exists, else the tile kernels'
+// default.  Mixed: 4 cells a thread, CTAs of 128 threads along x and 256 along y and z; one of 512 has an SM to
+// itself and nothing to hide its barriers behind (256^3, at the time: x 324 us with 64 to 128 threads, 355 with
+// 256, 425 with 512; y 504 us with 4 pencils in 256 threads, 534 with 8 in 512).  FP64: 2 cells a thread while two CTAs'
+// exchange records fit an SM (192 threads; 96^3 x 50 us, y 57 us), else 4 (96^3: 62 and 65 us; 128^3 y: 137 us,
+// with 2 cells in 256 threads 199 us).
 PencilCfg choose_fluid(const Geom& g, int d, size_t elem, const PencilCfg& tile) {
-    if (elem == 8) return tile;
     std::vector<PencilCfg> c = seg_candidates(g, d, elem);
-    const PencilCfg* best = default_segments(c, d);
+    // (longer pencils keep 4: their CTAs have the warps, and tubes of an ensemble fill the chip together)
+    const PencilCfg* best = small_grid(g) && g.n[d] <= 256 ? default_segments(c, g, d, elem, 2, 128, 2.0) : nullptr;
+    if (!best && elem == 8) {
+        std::vector<PencilCfg> two;
+        for (const PencilCfg& p : c)
+            if (p.seg == 2 && p.NT <= 192 && p.CL == 1 && (d == 0 || p.Wb >= 4)) two.push_back(p);
+        best = default_segments(two, g, d, elem, 2, 128, 1.0);
+        if (best) return *best;
+    }
+    if (!best) best = default_segments(c, g, d, elem, 4, d == 0 ? 128 : 256, 2.0);
     return best ? *best : tile;
 }
 
@@ -750,30 +741,50 @@ PencilLaunch pencil_launch(const img_ctx* ctx, const PencilCfg& pcf, int d, size
     return L;
 }
 
+// The rounding of a segment launch (FP32; FP64 has form 1 alone).  Form 2 rounds every sum as the pencil-tile
+// kernels do, form 1 differs from it in the last bit of the fluxes' B terms and of every fourth cell's half step
+// (seg_flux, seg_predict).  A grid's steps have to keep rounding alike, for FP32 differences grow with the flow's own
+// instabilities (a 64^2 vortex: from the last bit to 2e-5 in 60 steps, 256^3 shear layers past 1e-3 in 120), so the form
+// follows the grid, not the tiling.  Form 1: artificial viscosity; tilings that
+// the autotuner or img_set_tiling picked; pencils of whole
+// 4-cell segments that make CTAs of 64 to 512 threads (x: a power of two up to 32 of them or a multiple of 32, or 64 and
+// more with const ends; y and z: 8 pencils side by side); whole pencils of one thread across y and z.  Form 2: the
+// others, which the tile kernels can serve too.
+int flux_form(const Geom& g, int d, size_t elem, const img_config& c, bool fade, bool picked) {
+    if (fade) return 2;
+    if (elem == 8 || picked || c.viscosity_type != IMG_VISC_NONE) return 1;
+    const int N = g.n[d], S = (N + 3) / 4;
+    const long long ncol = g.ncell / N;
+    const bool fits_x = S % 32 == 0 || (S <= 32 && 32 % S == 0);
+    auto block = [&](int S1, int lo, int hi) {   // some power of two of pencils in [lo, hi] makes such a CTA
+        for (int Wb = lo; Wb <= hi && Wb * S1 <= 512 && (Wb == 1 || Wb / 2 < ncol); Wb *= 2)
+            if (Wb * S1 >= 64 && Wb * S1 % 32 == 0) return true;
+        return false;
+    };
+    if (N % 4 == 0 && (d != 0 || fits_x) && block(S, d == 0 ? 1 : 8, d != 0 && S == 1 ? 512 : 32)) return 1;
+    if (d != 0) return (N == 2 || N == 3 || N == 4 || N == 8) && block(1, 4, 512) ? 1 : 2;
+    const bool const_ends = c.bc_modes[CLS_MASS][0][d] == IMG_BC_CONST && c.bc_modes[CLS_MASS][1][d] == IMG_BC_CONST;
+    return S >= 64 && S <= 2048 && (N % 4 == 0 || const_ends) ? 1 : 2;
+}
+
 template <typename T>
 int launch_fluid(img_ctx* ctx, int d, bool cfl) {
     FluidArgs a{};
     const img_config& c = ctx->cfg;
-    // the segment kernel takes the steady sweeps of single-CTA pencils whose ends are circ or const for
-    // all fluid classes; stored-edge capture (a run's first sweeps), fade and other ends take the tile
-    // kernels
+    // the segment kernel takes the sweeps whose ends are circ, const or fade, the same for all fluid classes
+    // (fade: pencils of one CTA, 2 or 4 cells per thread); stored-edge capture (a run's first sweep) and
+    // other ends take the tile kernels
     const bool fade = fade_on(c, d, CLS_MASS, CLS_ENER);
     const bool init = ctx->init_store || ctx->init_flux;
-    bool seg_ok = ctx->pcfg[0][d].seg && !init && !fade;
+    const PencilCfg& ps = ctx->pcfg[0][d];
+    bool seg_ok = ps.seg && !init && !(fade && (ps.CL > 1 || (ps.seg != 2 && ps.seg != 4)));
     for (int k = 0; k < 3; ++k)
-        for (int side = 0; side < 2; ++side) {
-            const int m = c.bc_modes[k][side][d];
-            if ((m != IMG_BC_CIRC && m != IMG_BC_CONST) || m != c.bc_modes[CLS_MASS][side][d]) seg_ok = false;
-        }
+        for (int side = 0; side < 2; ++side)
+            if (!copy_ghost_mode(c.bc_modes[k][side][d]) || c.bc_modes[k][side][d] != c.bc_modes[CLS_MASS][side][d]) seg_ok = false;
     // with artificial viscosity the tiling is always a segment one and every swept end circ or const
     // (img_create and img_set_tiling see to it), so no stored edge is ever read: the first sweeps too
     const bool visc = c.viscosity_type != IMG_VISC_NONE;
     if (visc) seg_ok = true;
-    // a ragged last segment (cluster forms) supports const ends only
-    const bool clu = seg_cluster_form(ctx->pcfg[0][d], ctx->g.n[d]);
-    if (clu && ctx->g.n[d] % ctx->pcfg[0][d].seg != 0)
-        for (int side = 0; side < 2; ++side)
-            if (c.bc_modes[CLS_MASS][side][d] != IMG_BC_CONST) seg_ok = false;
     const PencilCfg& pcf = (seg_ok || !ctx->pcfg[0][d].seg) ? ctx->pcfg[0][d] : ctx->pcfg_tile[d];
     a.sg = sweep_geom(ctx, d, pcf);
     for (int v = 0; v < NQ; ++v) a.q[v] = ctx->q[v];
@@ -782,6 +793,7 @@ int launch_fluid(img_ctx* ctx, int d, bool cfl) {
     a.minmass = c.minmass;
     a.minmass_out = ctx->fade_mask ? -HUGE_VAL : c.minmass;   // the point-fade pass clamps
     a.dx = c.dgrid[d];
+    a.inv_dx = 1.0 / c.dgrid[d];
     a.limiter = c.limiter[d];
     for (int k = 0; k < 4; ++k) {
         a.mode[k][0] = c.bc_modes[k][0][d];
@@ -807,10 +819,11 @@ int launch_fluid(img_ctx* ctx, int d, bool cfl) {
         a.vc1sq = c1 * c1;
     }
     PencilLaunch L = pencil_launch<T>(ctx, pcf, d,
-                                      pcf.seg ? seg_fluid_smem_bytes<T>(pcf.NT, visc) : fluid_smem_bytes<T>(pcf.G * pcf.cpt, pcf.Wb),
+                                      pcf.seg ? seg_smem(sizeof(T), pcf.NT, pcf.Wb, visc, fade)
+                                              : fluid_smem_bytes<T>(pcf.G * pcf.cpt, pcf.Wb),
                                       1, fade);
     L.seg = pcf.seg;
-    L.clu = seg_cluster_form(pcf, ctx->g.n[d]);
+    L.clu = seg_cluster_form(pcf);
     // copy ghosts: single-CTA pencils, one circ, const or fade mode per side shared by the fluid classes
     L.cg = pcf.CL == 1;
     for (int k = 0; k < 3; ++k)
@@ -820,11 +833,13 @@ int launch_fluid(img_ctx* ctx, int d, bool cfl) {
         }
     L.init = a.init_store || a.init_flux;   // first sweeps: the stored-edge capturing kernel
     if (L.seg) L.cg = true;                  // segment kernels index their ghosts directly
+    const int form = L.seg ? flux_form(ctx->g, d, sizeof(T), c, fade, pcf.picked) : 1, mhd = ctx->mhd ? form : 0;
+    a.round_cells = sizeof(T) == 4 && form == 1 ? (ctx->g.n[d] < 4 ? ctx->g.n[d] : 4) : 0;
     if (ctx->rec) {
         OpRec r{};
         r.kind = OP_FLUID;
         r.elem = sizeof(T);
-        r.mhd = ctx->mhd != 0;
+        r.mhd = mhd;
         r.L = L;
         r.fa = a;
         ctx->rec->push_back(r);
@@ -832,7 +847,7 @@ int launch_fluid(img_ctx* ctx, int d, bool cfl) {
         ctx->init_flux = false;
         return IMG_OK;
     }
-    cudaError_t le = launch_fluid_sweep<T>(a, L, ctx->mhd != 0);
+    cudaError_t le = launch_fluid_sweep<T>(a, L, mhd);
     if (le != cudaSuccess)
         return fail(ctx, IMG_ERR_CUDA, "fluid sweep launch (dim %d, grid %u, block %u, smem %zu, cluster %d): %s", d,
                     L.grid_x, L.block, L.smem, L.cluster, cudaGetErrorString(le));
@@ -1804,9 +1819,15 @@ int img_set_state(img_ctx* ctx, const double* mass, const double* mom, const dou
     ctx->state_set = true;
     ctx->cfl_valid = false;
     // new FluidArray/MagnetArray objects: their InitializedArrays take edges at first assignment
-    ctx->init_store = ctx->init_flux = true;
+    // (in FP64 only where some boundary stores one, trans or wall; the mixed form's first sweeps always take the
+    // capturing kernels, whose rounding its later steps go on from)
+    bool captures = ctx->elem == 4;
+    for (const auto& cls : ctx->cfg.bc_modes)
+        for (const auto& side : cls)
+            for (int m : side) captures = captures || stateful(m);
+    ctx->init_store = ctx->init_flux = captures;
     for (auto& r : ctx->init_mag)
-        for (auto& v : r) v = true;
+        for (auto& v : r) v = captures;
     return IMG_OK;
 }
 
@@ -2179,7 +2200,7 @@ int img_totals(img_ctx* ctx, double out[8]) {
 struct BatchItem {            // one batched launch
     int kind = 0, elem = 0;
     int op = 0;               // index of the members' launch it batches (the groups of one op run side by side)
-    bool mhd = false;
+    int mhd = 0;
     PencilLaunch L{};         // pencil kernels: the shared shape; grid_x = CTAs of all members
     unsigned blocks = 0;      // pointwise kernels: blocks of all members
     size_t args_off = 0, map_off = 0;
@@ -2811,6 +2832,7 @@ int img_autotune(img_ctx* ctx, int trials) {
                     best = cand;
                 }
             }
+            best.picked = true;
             ctx->pcfg[kind][d] = best;
             std::lock_guard<std::mutex> lock(g_tune_mu);
             g_tuned[tune_key(kind, ctx->g, d, ctx->elem, ctx->cfg)] = best;
@@ -2843,6 +2865,7 @@ int img_set_tiling(img_ctx* ctx, int dim, const int cfg[7]) {
             (c.seg != 0) != (cfg[6] != 0))
             continue;
         c.nqc = nqc;
+        c.picked = true;
         if (c.seg) {
             ctx->pcfg[kind][d] = c;
             if (kind == 1) ctx->pcfg[2][d] = c;

@@ -36,6 +36,9 @@ template <typename V, typename T> __device__ __forceinline__ V v_dup(T x) {
     else return x;
 }
 
+__device__ __forceinline__ F2 v_pick(bool c, F2 a, F2 b) { a.v = c ? a.v : b.v; return a; }
+template <typename T> __device__ __forceinline__ T v_pick(bool c, T a, T b) { return c ? a : b; }
+
 // The limiter correction of each lane.  Van Leer: dL dR / (dL + dR) where the product is positive, else 0.
 // A positive FP32 product keeps |dL + dR| above 2^-75, so the one-instruction reciprocal never sees a
 // subnormal (which its .ftz form would flush).

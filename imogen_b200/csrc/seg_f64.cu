@@ -2,7 +2,7 @@
 #include "seg_impl.cuh"
 
 namespace img {
-template cudaError_t launch_fluid_seg<double>(const FluidArgs&, const PencilLaunch&, bool);
-template cudaError_t launch_fluid_seg_batch<double>(const FluidArgs*, const BlockMap*, const PencilLaunch&, bool);
+template cudaError_t launch_fluid_seg<double>(const FluidArgs&, const PencilLaunch&, int);
+template cudaError_t launch_fluid_seg_batch<double>(const FluidArgs*, const BlockMap*, const PencilLaunch&, int);
 template cudaError_t fluid_seg_attributes<double>(int);
 }  // namespace img

@@ -1,82 +1,87 @@
 // Segment form of the fused fluid sweep (fluid/relaxingFluid.m:16-73, fluid/wFluidFlux.m:14-44,
-// pressure/pressure.m:23-64, flux/*Limiter.m) for pencils that fit one CTA with circ or const ends.
+// pressure/pressure.m:23-64, flux/*Limiter.m) for pencils with circ, const or fade ends.
 //
-// Each thread owns C consecutive cells of a pencil (a "segment"), so every stencil neighbour inside a
-// segment is a register; only the cells at the two ends of a segment are exchanged, through shared
-// memory, and the exchanges ride on the two barriers that the pencil maxima need anyway:
+// Each thread owns C consecutive cells of a pencil (a "segment"; the last one may be shorter), so every
+// stencil neighbour inside a segment is a register; only the cells at the two ends of a segment are
+// exchanged, through shared memory, and the exchanges ride on the two barriers that the pencil maxima
+// need anyway:
 //   stage 1  load the segment (128-bit loads along x), 'totsnd' pressure, freezing-speed candidate and
 //            the flux numerators F (w = F / c_f) of every cell; publish (u, F) of the first and last
 //            cell; barrier; c_f = pencil max.
-//   stage 2  predictor half step with R = (u + F/c_f)/2, L = (u - F/c_f)/2 (relaxingFluid.m:30-39);
-//            pressure, speed and F of the half-step state; publish (u*, F*) of the first two and last
-//            two cells; barrier; c_f* = pencil max.
-//   stage 3  corrector fluxes R*, L* over the segment and the two neighbour cells each side, the TVD
-//            limiter (relaxingFluid.m:57-62) -- the limited values of the neighbour cells next to the
-//            segment are computed here as well, from the published cells -- and the update
-//            (relaxingFluid.m:64-71); store; fused CFL maxima on the last sweep of a step.
+//   stage 2  predictor half step (relaxingFluid.m:30-39); pressure, speed and F of the half-step state;
+//            publish (u*, F*) of the first two and last two cells; barrier; c_f* = pencil max.
+//   stage 3  corrector fluxes over the segment and the two neighbour cells each side, the TVD limiter
+//            (relaxingFluid.m:57-62) -- the limited values of the neighbour cells next to the segment are
+//            computed here as well, from the published cells -- and the update (relaxingFluid.m:64-71);
+//            store; fused CFL maxima on the last sweep of a step.
+// R = (u + F/c_f)/2 and L = (u - F/c_f)/2 take one FMA each (the predictor leaves the 2 to the update).  In the mixed form two variables at a time go through the
+// packed FP32 instructions (lanes.cuh).
+// Fade ends (fade_shift.m) blend every shifted array near the ends toward the shifted end values: those
+// launches (FADE) form the shifted values cell by cell, take the ends' rows from a small anchor set and
+// exchange the limited fluxes behind one more barrier.
 // With artificial viscosity (fluid/ArtificialViscosity.m) stages 1 and 2 each publish the viscosity
 // exchange set with the pencil maximum, then compute the viscous pressure and F and publish (u, F)
 // behind one more barrier: four barriers instead of two.
-// Per cell the formulas are those of the pencil-tile kernels (fluid_sweep.cuh); the momentum and
-// cell-centred B are held in sweep-rotated order (the component along the sweep first), so sums over
-// components run in that order, and the compiler may contract differently into FMAs: the two kernel
-// families agree to round-off, not bit for bit.  The limiter is fixed per launch and compiled into the
-// corrector (seg_correct).
+// Per cell the operations are those of the pencil-tile kernels (fluid_sweep.cuh) in the same order; the momentum
+// and cell-centred B are held in sweep-rotated order (the component along the sweep first).  The FMAs are written
+// out (the unit is compiled without implicit ones), so results do not depend on the tiling.  MHD = 2 sums and
+// rounds the B terms of the fluxes as the pencil-tile kernels do, MHD = 1 in rotated order (seg_flux).
 //
 // Thread placement (SweepGeom with G = S segments per pencil, RC = N): along x the S threads of a
 // pencil are consecutive (thread t = b*S + s), along y and z the Wb pencils of the CTA are (t = s*Wb +
-// b), so global loads and stores stay coalesced along x.  Pencil ends: a circ end's neighbour segment
-// is the pencil's other end; a const end's ghost is the end cell itself (constant_shift.m), applied to
-// every shifted array, the limited fluxes included.
+// b), so global loads and stores stay coalesced along x; threads past the last segment idle.  A pencil
+// along x may span the CTAs of a cluster (CLU; segment s = rank*NT + t), whose exchanges then read the
+// neighbours' shared memory through DSMEM.  Pencil ends: a circ end's neighbour is the pencil's other end;
+// a const (or fade) end's ghost is the end cell itself (constant_shift.m), applied to every shifted array,
+// the limited fluxes included.
 #pragma once
 
 #include <type_traits>
 
 #include "fluid_sweep.cuh"
+#include "lanes.cuh"
 
 namespace img {
 
 // FP64 words per thread of the artificial-viscosity exchange set (seg_visc_publish).
 constexpr int VISC_ROWS = 9;
 
-// Words per thread of the two exchange sets and of the pencil maxima: (u, F) of 2 cells, (u*, F*) of
-// 4 cells, and 2 per-warp maxima slots of 32 columns; with artificial viscosity the FP64 viscosity
-// exchange set after them.
+// Shared memory: per thread the exchange records, (u, F) of 2 cells and (u*, F*) of 4 cells, 10 values
+// each; two pencil maxima per pencil; then the FP64 viscosity exchange set, or with fade ends the anchors
+// (4 rows of 10 values per pencil and stage, 4 of 5 for the limited fluxes).
 template <typename T>
-__host__ __device__ inline size_t seg_fluid_smem_bytes(int NT, bool visc = false) {
-    return sizeof(T) * ((size_t)60 * NT + 2 * (size_t)(NT / 32) * 32) + (visc ? sizeof(double) * VISC_ROWS * NT : 0);
+__host__ __device__ inline size_t seg_fluid_smem_bytes(int NT, int Wb, bool visc = false, bool fade = false) {
+    return sizeof(T) * (size_t)60 * NT + 16 * (size_t)Wb + (visc ? sizeof(double) * VISC_ROWS * NT : 0) +
+           (fade ? sizeof(T) * (size_t)100 * Wb : 0);
 }
 
 // Placement of one thread in the segment layout.
 struct SegPos {
     int b, s;            // pencil within the CTA, segment within the pencil
-    int rank = 0;        // cluster rank (one pencil per cluster)
+    int rank;            // cluster rank (one pencil per cluster)
     bool colok;          // the pencil exists (the last CTA may hold fewer than Wb) and so does the segment
-    long long base;      // offset of the pencil's row 0
-    // One pencil along x over the CL CTAs of a cluster (CL = 1: one CTA), S = ceil(N / C) segments of
-    // which rank r holds r * NT .. r * NT + NT - 1; threads past the last segment idle.
-    __device__ __forceinline__ void init_cluster(const SweepGeom& g, unsigned vblock) {
-        const unsigned blk = g.div_cl.div(vblock);
-        rank = (int)(vblock - blk * (unsigned)g.CL);
-        b = 0;
-        s = rank * g.NT + (int)threadIdx.x;
-        colok = s < g.G && (long long)blk < g.ncol;
-        const unsigned c = colok ? blk : 0u;
-        const int c2 = (int)g.div_n1.div(c);
-        const int c1 = (int)(c - (unsigned)c2 * (unsigned)g.n1);
-        base = c1 * g.s1 + (long long)c2 * g.s2;
-    }
+    int base;            // offset of the pencil's row 0 (grids have fewer than 2^31 cells)
+    template <bool CLU>
     __device__ __forceinline__ void init(const SweepGeom& g, unsigned vblock) {
-        const int t = threadIdx.x;
-        const unsigned q = g.div_lanes.div((unsigned)t);   // t / S (x) or t / Wb (y, z)
-        if (g.d == 0) { b = (int)q; s = t - b * g.G; }
-        else { s = (int)q; b = t - s * g.Wb; }
-        const int col = (int)(vblock * (unsigned)g.Wb + (unsigned)b);
-        colok = col < g.ncol;
+        int t = threadIdx.x;
+        unsigned blk = vblock;
+        rank = 0;
+        if constexpr (CLU) {   // one pencil over the CL CTAs of a cluster (CL = 1: one CTA)
+            blk = g.div_cl.div(vblock);
+            rank = (int)(vblock - blk * (unsigned)g.CL);
+            b = 0;
+            s = t + rank * g.NT;
+        } else {
+            const unsigned q = g.div_lanes.div((unsigned)t);   // t / S (x) or t / Wb (y, z)
+            if (g.d == 0) { b = (int)q; s = t - b * g.G; }
+            else { s = (int)q; b = t - s * g.Wb; }
+        }
+        const int col = (int)(blk * (unsigned)g.Wb + (unsigned)b);
+        colok = col < (int)g.ncol && b < g.Wb && s < g.G;
         const unsigned c = colok ? (unsigned)col : 0u;
         const int c2 = (int)g.div_n1.div(c);
         const int c1 = (int)(c - (unsigned)c2 * (unsigned)g.n1);
-        base = c1 * g.s1 + (long long)c2 * g.s2;
+        base = c1 * (int)g.s1 + c2 * (int)g.s2;
     }
 };
 
@@ -128,49 +133,104 @@ __device__ __forceinline__ void seg_store(void* p, long long o, long long sd, bo
     for (int k = 0; k < C; ++k) a[(long long)k * sd] = v[k];
 }
 
-// The flux numerators F of wFluidFlux.m:31-44 (w = F * (1/c_f)) for one cell whose momentum and
-// cell-centred B are held in sweep-rotated order (component 0 along the sweep): the mixed form with the
-// one-instruction FP32 reciprocal of rho, FP64 with the IEEE reciprocal (the operations of wflux).
-template <typename T>
-__device__ __forceinline__ void flux_num_rot(const T u[5], const T bb[3], T press, T F[5]) {
-    T ir;
-    if constexpr (sizeof(T) == 4) ir = rcp_approx(u[0]);
-    else ir = T(1) / u[0];
-    const T velocity = u[1] * ir;
-    F[0] = u[1];
-    F[4] = velocity * (u[4] + press) - bb[0] * (bb[0] * u[1] + bb[1] * u[2] + bb[2] * u[3]) * ir;
-    F[1] = velocity * u[1] + press - bb[0] * bb[0];
-    F[2] = velocity * u[2] - bb[0] * bb[1];
-    F[3] = velocity * u[3] - bb[0] * bb[2];
-}
-
-// 'totsnd' pressure and the freezing-speed candidate |p_X / rho| + c_s of one cell (rotated order).
-template <typename T>
-__device__ __forceinline__ T press_speed_rot(double G, const T u[5], double msq, T& p) {
-    if constexpr (sizeof(T) == 4) {
-        PressOutF o = pressure_totsnd_mixed(G, u[0], u[1], u[2], u[3], u[4], msq);
-        p = o.p;
-        return fabsf(u[1] * rcp_approx(u[0])) + o.cs;
+// Own cells of an array: vector accesses where the segments allow (vec), else cell by cell; past the
+// pencil's end (a ragged last segment, idle threads) `fill`, and nothing stored.
+// ONCE: the strided cells of y and z sweeps are loaded past the L1 cache (nobody reads them again, and their
+// 32-byte rows would each take a 128-byte line from what does come back).
+template <typename T, int C, bool ONCE = false>
+__device__ __forceinline__ void win_load(const void* ptr, int o, int sd, bool vec, int nown, T fill, T (&out)[C]) {
+    const T* p = reinterpret_cast<const T*>(ptr);
+    if (vec && nown == C) {
+        seg_load<T, C>(p, o, 1, true, out);
+    } else if (ONCE && sd != 1) {
+#pragma unroll
+        for (int k = 0; k < C; ++k) out[k] = k < nown ? __ldcg(p + (o + k * sd)) : fill;
     } else {
-        PressOut o = pressure_totsnd(G, u[0], u[1], u[2], u[3], u[4], msq);
-        p = o.p + 0.0;   // + viscosity.solve ('empty' -> 0)
-        return fabs(u[1] * (1.0 / u[0])) + o.cs;
+#pragma unroll
+        for (int k = 0; k < C; ++k) out[k] = k < nown ? p[o + k * sd] : fill;
+    }
+}
+template <typename T, int C>
+__device__ __forceinline__ void win_store(void* ptr, int o, int sd, bool vec, int nown, const T (&v)[C]) {
+    T* p = reinterpret_cast<T*>(ptr);
+    if (vec && nown == C) {
+        seg_store<T, C>(p, o, 1, true, v);
+    } else {
+#pragma unroll
+        for (int k = 0; k < C; ++k)
+            if (k < nown) p[o + k * sd] = v[k];
     }
 }
 
-// The same, also returning the 'totsnd' sound speed (the Neumann-Richtmyer viscosity reads it).
-template <typename T>
-__device__ __forceinline__ T press_speed_rot(double G, const T u[5], double msq, T& p, T& cs) {
-    if constexpr (sizeof(T) == 4) {
-        PressOutF o = pressure_totsnd_mixed(G, u[0], u[1], u[2], u[3], u[4], msq);
-        p = o.p;
-        cs = o.cs;
-        return fabsf(u[1] * rcp_approx(u[0])) + o.cs;
+// Constants of the 'totsnd' pressure (pressure.m:23-64) from gamma.
+struct SegPressure {
+    double g, g1, half_g1, p_ms;
+    __device__ __forceinline__ explicit SegPressure(double G) : g(G), g1(G - 1.0), half_g1((G - 1.0) * 0.5), p_ms(0.5 * (2.0 - G)) {}
+    // P and rho c_s^2 from p0 = (G-1)(E - rho v^2/2) and msq = B^2
+    template <int MSQ>
+    __device__ __forceinline__ void totals(double p0, double msq, double& pt, double& c2) const {
+        if constexpr (MSQ) {
+            c2 = fma(2.0, msq, g * fma(-half_g1, msq, p0));
+            pt = fma(p_ms, msq, p0);
+        } else {
+            c2 = g * p0;
+            pt = p0;
+        }
+    }
+};
+
+// 'totsnd' pressure, sound speed, 1/rho and the freezing-speed candidate |p_X / rho| + c_s of one cell
+// (rotated order; msq = B^2 of the cell-centred components without isZero).  Mixed form: FP64 throughout,
+// with 1/rho from the one-instruction FP32 estimate refined by one FP64 Newton step; the sound speed's
+// square root is taken in FP32.
+template <int MSQ>
+__device__ __forceinline__ float seg_pressure(const SegPressure& k, const float (&u)[5], double msq, float& p, float& cs,
+                                              float& ir) {
+    ir = rcp_approx(u[0]);
+    const double e0 = (double)ir;
+    const double inv = e0 * fma(-(double)u[0], e0, 2.0);
+    const double px = u[1], py = u[2], pz = u[3];
+    const double psq = fma(pz, pz, fma(px, px, py * py));
+    double c2, pt;
+    k.totals<MSQ>(k.g1 * fma(-(0.5 * psq), inv, (double)u[4]), msq, pt, c2);
+    cs = sqrt_approx(fabsf((float)(c2 * inv)));
+    p = pt < 0 ? 0.f : (float)pt;
+    return fabsf(u[1] * ir) + cs;
+}
+template <int MSQ>
+__device__ __forceinline__ double seg_pressure(const SegPressure& k, const double (&u)[5], double msq, double& p, double& cs,
+                                               double& ir) {
+    ir = recip(u[0]);
+    const double psq = fma(u[3], u[3], fma(u[1], u[1], u[2] * u[2]));
+    double c2, pt;
+    k.totals<MSQ>(k.g1 * fma(-(0.5 * psq), ir, u[4]), msq, pt, c2);
+    cs = sqrt_goldschmidt(fabs(c2 * ir));
+    p = pt < 0 ? 0.0 : pt;
+    return fabs(u[1] * ir) + cs;
+}
+
+// The flux numerators F of wFluidFlux.m:31-44 (w = F / c_f) for one cell (rotated order).  MHD = 2: B.p is summed in
+// the order x, y, z, and the transverse momentum fluxes round v p before they take B B off it, as the pencil-tile
+// kernels do; MHD = 1: B.p in rotated order, B B rounded first.
+template <typename T, int MHD>
+__device__ __forceinline__ void seg_flux(int d, bool tile, const T (&u)[5], const T (&bb)[3], T press, T ir, T (&F)[5]) {
+    const T velocity = u[1] * ir;
+    F[0] = u[1];
+    if constexpr (MHD) {
+        T dot;
+        if (MHD == 1 || d == 0) dot = v_fma(bb[2], u[3], v_fma(bb[0], u[1], bb[1] * u[2]));
+        else if (d == 1) dot = v_fma(bb[2], u[3], v_fma(bb[1], u[2], bb[0] * u[1]));
+        else dot = v_fma(bb[0], u[1], v_fma(bb[1], u[2], bb[2] * u[3]));
+        F[4] = v_fma(velocity, u[4] + press, -((bb[0] * dot) * ir));
+        if (MHD == 2) F[1] = v_fma(-bb[0], bb[0], velocity * u[1] + press);
+        else F[1] = v_fma(velocity, u[1], press) - bb[0] * bb[0];
+        F[2] = MHD == 2 ? v_fma(-bb[0], bb[1], velocity * u[2]) : v_fma(velocity, u[2], -(bb[0] * bb[1]));
+        F[3] = MHD == 2 ? v_fma(-bb[0], bb[2], velocity * u[3]) : v_fma(velocity, u[3], -(bb[0] * bb[2]));
     } else {
-        PressOut o = pressure_totsnd(G, u[0], u[1], u[2], u[3], u[4], msq);
-        p = o.p;
-        cs = o.cs;
-        return fabs(u[1] * (1.0 / u[0])) + o.cs;
+        F[4] = velocity * (u[4] + press);
+        F[1] = tile ? velocity * u[1] + press : v_fma(velocity, u[1], press);
+        F[2] = velocity * u[2];
+        F[3] = velocity * u[3];
     }
 }
 
@@ -285,108 +345,116 @@ __device__ __forceinline__ T visc_add(T p, double q) {
     else return __dadd_rn(p, q);
 }
 
-// Corrector (relaxingFluid.m:52-71) of one variable over a segment: R* = (u* + F*/c_f*)/2 and
-// L* = (u* - F*/c_f*)/2 at cells -2 .. C+1 (neighbour cells from the published exchange set X2), the
-// TVD limiter at cells -1 .. C (only those the update reads), and the update of the C own cells.
-// LIM: the launch's limiter (flux/*Limiter.m), fixed at compile time.  X2l/X2r: the exchange sets that
-// hold the left and right neighbour segments (another CTA's, through DSMEM, across a cluster).
-// nown < C: a ragged last segment with a const end after cell nown - 1 (its cells beyond hold copies of
-// that cell's state), whose limited L takes the end cell's value one cell past it.
-template <typename T, int C, int LIM>
-__device__ __forceinline__ void seg_correct(const T (&u)[C], const T (&us)[C], const T (&Fs)[C], const T* X2l,
-                                            const T* X2r, int NT, int lt, int rt, bool lo_own, bool hi_own, T ics,
-                                            T ffc, T (&unew)[C], int nown = C) {
-    const T* X2v = X2l;
-    T Rs[C + 4], Ls[C + 4];
+// ---- exchange records ---------------------------------------------------------------------------------
+// The 10 values (u, F) of one cell, `slots` records per thread, in parts by the variables that are worked on
+// together: 16 bytes of (u, F) of two FP32 variables or one FP64 variable (8 for the fifth FP32 one), the same
+// part of consecutive threads' records on consecutive 16 bytes.
+template <typename T>
+__host__ __device__ constexpr int seg_rec_bytes() { return 10 * (int)sizeof(T); }
+
+__device__ __forceinline__ void rec_put(unsigned char* X, int slots, int slot, int NT, int t, const float (&u)[5],
+                                        const float (&F)[5]) {
+    const int i = slot * NT + t, n = slots * NT;
+    reinterpret_cast<float4*>(X)[i] = make_float4(u[0], u[1], F[0], F[1]);
+    reinterpret_cast<float4*>(X)[n + i] = make_float4(u[2], u[3], F[2], F[3]);
+    reinterpret_cast<float2*>(X)[4 * n + i] = make_float2(u[4], F[4]);
+}
+__device__ __forceinline__ void rec_put(unsigned char* X, int slots, int slot, int NT, int t, const double (&u)[5],
+                                        const double (&F)[5]) {
+    const int i = slot * NT + t, n = slots * NT;
+    double2* P = reinterpret_cast<double2*>(X);
 #pragma unroll
-    for (int k = 0; k < C; ++k) {
-        const T w = Fs[k] * ics;
-        Rs[k + 2] = T(0.5) * (us[k] + w);
-        Ls[k + 2] = T(0.5) * (us[k] - w);
-    }
-    if (lo_own) {
-        Rs[1] = Rs[2]; Ls[1] = Ls[2];
-        Rs[0] = Rs[2]; Ls[0] = Ls[2];
-    } else {   // X2v holds [u*, F*] x [cell 0, cell 1, cell C-2, cell C-1] at strides of 5*NT
-        const T u1 = X2v[30 * NT + lt], w1 = X2v[35 * NT + lt] * ics;   // left's last cell
-        const T u2 = X2v[20 * NT + lt], w2 = X2v[25 * NT + lt] * ics;   // left's cell C-2
-        Rs[1] = T(0.5) * (u1 + w1); Ls[1] = T(0.5) * (u1 - w1);
-        Rs[0] = T(0.5) * (u2 + w2); Ls[0] = T(0.5) * (u2 - w2);
-    }
-    if (hi_own) {
-        Rs[C + 2] = Rs[C + 1]; Ls[C + 2] = Ls[C + 1];
-        Rs[C + 3] = Rs[C + 1]; Ls[C + 3] = Ls[C + 1];
+    for (int v = 0; v < 5; ++v) P[v * n + i] = make_double2(u[v], F[v]);
+}
+// Variables v .. v + M - 1 (one part) of record i.
+template <int v, int M>
+__device__ __forceinline__ void rec_part(const unsigned char* X, int slots, int i, int NT, float (&u)[M], float (&F)[M]) {
+    const int n = slots * NT;
+    if constexpr (M == 2) {
+        const float4 a = reinterpret_cast<const float4*>(X)[(v / 2) * n + i];
+        u[0] = a.x; u[1] = a.y; F[0] = a.z; F[1] = a.w;
     } else {
-        const T u1 = X2r[rt], w1 = X2r[5 * NT + rt] * ics;                // right's first cell
-        const T u2 = X2r[10 * NT + rt], w2 = X2r[15 * NT + rt] * ics;      // right's cell 1
-        Rs[C + 2] = T(0.5) * (u1 + w1); Ls[C + 2] = T(0.5) * (u1 - w1);
-        Rs[C + 3] = T(0.5) * (u2 + w2); Ls[C + 3] = T(0.5) * (u2 - w2);
+        static_assert(v == 4, "the fifth variable stands alone");
+        const float2 a = reinterpret_cast<const float2*>(X)[4 * n + i];
+        u[0] = a.x; F[0] = a.y;
     }
-    // limited R at cells -1 .. C-1 and limited L at cells 0 .. C (index j + 1)
-    T Rl[C + 1], Ll[C + 2];
+}
+template <int v, int M>
+__device__ __forceinline__ void rec_part(const unsigned char* X, int slots, int i, int NT, double (&u)[M], double (&F)[M]) {
+    static_assert(M == 1, "FP64 variables go one by one");
+    const double2 a = reinterpret_cast<const double2*>(X)[v * slots * NT + i];
+    u[0] = a.x; F[0] = a.y;
+}
+__device__ __forceinline__ void rec_get(const unsigned char* X, int slots, int i, int NT, float (&u)[5], float (&F)[5]) {
+    float a[2], b[2], c[1], d[1];
+    rec_part<0, 2>(X, slots, i, NT, a, b);
+    u[0] = a[0]; u[1] = a[1]; F[0] = b[0]; F[1] = b[1];
+    rec_part<2, 2>(X, slots, i, NT, a, b);
+    u[2] = a[0]; u[3] = a[1]; F[2] = b[0]; F[3] = b[1];
+    rec_part<4, 1>(X, slots, i, NT, c, d);
+    u[4] = c[0]; F[4] = d[0];
+}
+__device__ __forceinline__ void rec_get(const unsigned char* X, int slots, int i, int NT, double (&u)[5], double (&F)[5]) {
+    const int n = slots * NT;
+    const double2* P = reinterpret_cast<const double2*>(X);
 #pragma unroll
-    for (int j = -1; j < C; ++j) {
-        const T r = Rs[j + 2];
-        Rl[j + 1] = r + limiter_corr_t<LIM>(r - Rs[j + 1], Rs[j + 3] - r);
+    for (int v = 0; v < 5; ++v) {
+        const double2 a = P[v * n + i];
+        u[v] = a.x;
+        F[v] = a.y;
     }
-#pragma unroll
-    for (int j = 0; j <= C; ++j) {
-        const T l = Ls[j + 2];
-        Ll[j + 1] = l + limiter_corr_t<LIM>(Ls[j + 1] - l, l - Ls[j + 3]);
-    }
-    if (lo_own) Rl[0] = Rl[1];   // the limited flux's own const ghost
-    if (hi_own) Ll[C + 1] = Ll[C];
-    if (nown < C) {               // ragged end: the ghost one past cell nown - 1
-        T e = Ll[1];
-#pragma unroll
-        for (int j = 1; j < C; ++j)
-            if (j == nown) e = Ll[j];
-#pragma unroll
-        for (int j = 2; j <= C; ++j)
-            if (j == nown + 1) Ll[j] = e;
-    }
-#pragma unroll
-    for (int k = 0; k < C; ++k) unew[k] = u[k] - ffc * (Rl[k + 1] - Rl[k] + Ll[k + 1] - Ll[k + 2]);
 }
 
-// Pencil maximum of non-negative speeds in the segment layout.  publish: reduce over the lanes of the
-// pencil inside the warp and leave the warp's value in pm where a pencil spans warps; collect, after
-// a barrier, reduces those.  Along x the S segments of a pencil are consecutive lanes (S a power of
-// two below 32, or a multiple of 32); along y and z the lanes of pencil b are b, b + Wb, ... (Wb a
-// power of two, at most 32 when S > 1).  With S = 1 (a short pencil held whole by one thread, Wb up to
-// the CTA) the thread's own maximum is the pencil's.
-template <typename T>
-__device__ __forceinline__ T seg_max_publish(const SweepGeom& g, T v, T* pm) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned full = 0xffffffffu;
-    if (g.G == 1) return v;
-    if (g.d == 0) {
-        if (g.G >= 32) {
-            v = warp_max_nonneg(v);
-            if (lane == 0) pm[warp * 32] = v;
-        } else {
-            for (int o = g.G / 2; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(full, v, o));
-        }
-        return v;
-    }
-    for (int o = 16; o >= g.Wb; o >>= 1) v = fmax(v, __shfl_xor_sync(full, v, o));
-    if (lane < g.Wb) pm[warp * 32 + lane] = v;
-    return v;
-}
+// One neighbour's record: the exchange sets it lies in (another CTA's across a cluster) and its index.
+struct SegRef {
+    const unsigned char *X1, *X2;
+    int i1, i2;
+};
 
-template <typename T>
-__device__ __forceinline__ T seg_max_collect(const SweepGeom& g, int b, T wv, const T* pm) {
+// ---- pencil maxima ------------------------------------------------------------------------------------
+// Maximum of non-negative speeds over a pencil, kept as ordered bits per pencil in shared memory (zeroed
+// before the first barrier): each warp reduces what it can, then one shared atomic per pencil and warp
+// (per lane where a warp holds many short pencils).  One value to read after the barrier, where a table of
+// warp maxima took up to 16 loads and compares in every thread.
+__device__ __forceinline__ void seg_max_bits(unsigned* m, float v) { atomicMax(m, __float_as_uint(v + 0.0f)); }
+__device__ __forceinline__ void seg_max_bits(unsigned long long* m, double v) {
+    atomicMax(m, (unsigned long long)__double_as_longlong(v + 0.0));
+}
+template <typename T> struct SegBits { using U = unsigned long long; };
+template <> struct SegBits<float> { using U = unsigned; };
+__device__ __forceinline__ float seg_from_bits(unsigned b) { return __uint_as_float(b); }
+__device__ __forceinline__ double seg_from_bits(unsigned long long b) { return __longlong_as_double((long long)b); }
+
+template <typename T, bool CLU>
+__device__ __forceinline__ void seg_max_publish(const SweepGeom& g, const SegPos& sp, T v, typename SegBits<T>::U* m) {
     const int lane = threadIdx.x & 31;
-    if (g.G == 1) return wv;
-    if (g.d == 0) {
-        if (g.G < 32) return wv;
-        const int w0 = (b * g.G) >> 5, nw = g.G >> 5;
-        return warp_max_nonneg(lane < nw ? pm[(w0 + lane) * 32] : T(0));
+    const unsigned full = 0xffffffffu;
+    if (!CLU && g.G == 1) return;
+    if (CLU || (g.d == 0 && (g.G & 31) == 0)) {         // a warp's lanes belong to one pencil
+        v = warp_max_nonneg(v);
+        if (lane == 0 && sp.b < g.Wb) seg_max_bits(m + sp.b, v);
+    } else if (g.d != 0) {                               // lanes b, b + Wb, ... belong to pencil b
+        for (int o = 16; o >= g.Wb; o >>= 1) v = fmax(v, __shfl_xor_sync(full, v, o));
+        if (lane < g.Wb) seg_max_bits(m + sp.b, v);
+    } else {                                             // along x, segment counts of any size
+        const int b0 = __shfl_sync(full, sp.b, 0), b1 = __shfl_sync(full, sp.b, 31);
+        if (b0 == b1) {
+            v = warp_max_nonneg(v);
+            if (lane == 0 && sp.b < g.Wb) seg_max_bits(m + sp.b, v);
+        } else if (sp.b < g.Wb) {
+            seg_max_bits(m + sp.b, v);
+        }
     }
-    T m = T(0);
-    const int nw = g.NT >> 5;
-    for (int w = 0; w < nw; ++w) m = fmax(m, pm[w * 32 + b]);
-    return m;
+}
+template <typename T, bool CLU>
+__device__ __forceinline__ T seg_max_collect(const SweepGeom& g, const SegPos& sp, T own, typename SegBits<T>::U* m) {
+    if (!CLU && g.G == 1) return own;
+    if (CLU && g.CL > 1) {
+        T c = T(0);
+        for (int r = 0; r < g.CL; ++r) c = fmax(c, seg_from_bits(*cg::this_cluster().map_shared_rank(m, r)));
+        return c;
+    }
+    return seg_from_bits(m[sp.b < g.Wb ? sp.b : 0]);
 }
 
 // Stage barrier of the segment kernel: the cluster's where a pencil spans a cluster.
@@ -396,364 +464,695 @@ __device__ __forceinline__ void sp_sync(const SweepGeom& g) {
     else __syncthreads();
 }
 
-// Pencil maximum for one pencil over a cluster (init_cluster placement): publish leaves each warp's
-// maximum in pm; collect, after a barrier, reduces the CTA's warps and, with CL > 1, the CTAs' maxima
-// through DSMEM (slot `slot` of cm) behind one more cluster barrier.  All threads call both.
-template <typename T>
-__device__ __forceinline__ void clu_max_publish(T v, T* pm) {
-    v = warp_max_nonneg(v);
-    if ((threadIdx.x & 31) == 0) pm[(threadIdx.x >> 5) * 32] = v;
+// ---- predictor and corrector of one lane of variables --------------------------------------------------
+// Which of a segment's cells round the change of the half step before they add it (FluidArgs.round_cells = n: a
+// pencil's cells n - 1, 2 n - 1, ..., the energy excepted): END the last one, MID the fourth of 8; 0 none, 1 yes, 2 as
+// the launch says (round_cells is 4 in form 1 of the MHD fluxes wherever C is a multiple of 4, and 0 in form 2).
+template <typename T, int MHD, int C>
+__host__ __device__ constexpr int seg_round_mode() {
+    return sizeof(T) == 8 || MHD == 2 ? 0 : (MHD == 1 && C % 4 == 0 ? 1 : 2);
 }
 
+// Predictor (relaxingFluid.m:30-39): u and F at cells -1 .. C (index j + 1); ic = 1 / c_f, h = dt/dx c_f / 4.
+template <typename V, int C, int RND>
+__device__ __forceinline__ void seg_predict(const V (&u)[C + 2], const V (&F)[C + 2], V ic, V nic, V h, V nh, bool round4,
+                                            bool round_end, V (&us)[C]) {
+    V R[C + 1], L[C + 1];   // 2R at cells -1 .. C-1 (j + 1), 2L at cells 0 .. C (j)
+#pragma unroll
+    for (int j = 0; j <= C; ++j) {
+        R[j] = v_fma(F[j], ic, u[j]);
+        L[j] = v_fma(F[j + 1], nic, u[j + 1]);
+    }
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+        const V S = v_sub(v_add(v_sub(R[k + 1], R[k]), L[k]), L[k + 1]);
+        // (a product of pairs and a sum of pairs become one FMA; v_sub is an FMA itself, which keeps them apart)
+        if (RND == 1 && (k == C - 1 || k % 4 == 3)) {
+            us[k] = v_sub(u[k + 1], v_mul(h, S));
+        } else {
+            us[k] = v_fma(nh, S, u[k + 1]);
+            if (RND == 2 && (k == C - 1 || k % 4 == 3))
+                us[k] = v_pick(k == C - 1 ? round_end : round4, v_sub(u[k + 1], v_mul(h, S)), us[k]);
+        }
+    }
+}
+
+// Corrector (relaxingFluid.m:52-71): u*/2 and F* at cells -2 .. C+1 (index j + 2); ich = 1 / (2 c_f*), nh = -dt/dx c_f*.
+// (Not on 2R and 2L: the limiter's product would underflow elsewhere.)  The limited fluxes' own const ghosts: the
+// lower one copies cell 0's, the upper one that of end_k (the local cell at a const upper end, or C).
+template <typename V, int C, int LIM>
+__device__ __forceinline__ void seg_correct(const V (&u)[C], const V (&uh)[C + 4], const V (&Fs)[C + 4], V ich, V nich,
+                                            V nh, bool lo_end, int end_k, V (&unew)[C]) {
+    // R at cells j-1 .. j+1 and the difference below j (L likewise), rolled over j = -1 .. C
+    V R1 = v_fma(Fs[1], ich, uh[1]), L1, Rp, Lp, dR = v_sub(R1, v_fma(Fs[0], ich, uh[0])), dL, a;
+    L1 = v_fma(Fs[1], nich, uh[1]);
+#pragma unroll
+    for (int j = -1; j <= C; ++j) {
+        V Rl, Ll;
+        if (j < C) {
+            const V R2 = v_fma(Fs[j + 3], ich, uh[j + 3]), d = v_sub(R2, R1);
+            Rl = v_add(R1, v_limit<LIM>(dR, d));
+            R1 = R2;
+            dR = d;
+        }
+        {
+            const V L2 = v_fma(Fs[j + 3], nich, uh[j + 3]), d = v_sub(L2, L1);
+            if (j >= 0) Ll = v_sub(L1, v_limit<LIM>(dL, d));   // the limiters are odd
+            L1 = L2;
+            dL = d;
+        }
+        if (j >= 1) unew[j - 1] = v_fma(nh, v_sub(a, v_pick(j - 1 == end_k, Lp, Ll)), u[j - 1]);
+        if (j >= 0 && j < C) {
+            if (j == 0) Rp = v_pick(lo_end, Rl, Rp);
+            a = v_add(v_sub(Rl, Rp), Ll);
+        }
+        Rp = Rl;
+        Lp = Ll;
+    }
+}
+
+// Values of variables v, v + 1 (or v alone) as one lane.
+template <typename V, typename T> struct SegLane {
+    static constexpr int N = 1;
+    static __device__ __forceinline__ V get(T a, T) { return a; }
+    static __device__ __forceinline__ void put(V x, T& a, T&) { a = x; }
+};
+template <> struct SegLane<F2, float> {
+    static constexpr int N = 2;
+    static __device__ __forceinline__ F2 get(float a, float b) { return F2(a, b); }
+    static __device__ __forceinline__ void put(F2 x, float& a, float& b) { x.get(a, b); }
+};
+
+// Cell k (known at compile time) of the segment's variables.
+template <typename T, int C>
+__device__ __forceinline__ void cell(const T (&w)[5][C], int k, T (&c)[5]) {
+#pragma unroll
+    for (int v = 0; v < 5; ++v) c[v] = w[v][k];
+}
+// Whether cell k (known at compile time) is the n-th.  The comparison is kept opaque: seen together, a chain
+// of them over k becomes one access at a run-time index, which would move the whole array out of registers.
+__device__ __forceinline__ bool is_cell(int k, int n) {
+    asm("" : "+r"(n));
+    return k == n;
+}
+// What the stages need to know of a thread's place: its neighbours' records, the ends it sits at, its own cells.
+struct SegEnds {
+    bool round4, round_end;   // seg_predict
+    SegRef l1, l2, r1, r2;   // cells -1, -2 and the two past the last own cell
+    bool circ_lo, circ_hi;
+    bool solo;               // the whole pencil in this thread: its neighbours are its own cells
+    bool lo_own, hi_own;     // a const end below / above
+    int nown, NT;
+};
+
+// Predictor of variables v .. (one lane's) in place: u becomes u*.
+template <typename V, typename T, int C, int RND, int v>
+__device__ __forceinline__ void seg_predict_vars(const SegEnds& e, T (&u)[5][C], const T (&F)[5][C], T ic, T qh) {
+    using L = SegLane<V, T>;
+    constexpr int M = L::N, w = v + M - 1;
+    T ul[M], Fl[M], ur[M], Fr[M];
+    if (e.solo) {
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            ul[m] = e.circ_lo ? u[v + m][C - 1] : u[v + m][0];
+            Fl[m] = e.circ_lo ? F[v + m][C - 1] : F[v + m][0];
+            ur[m] = e.circ_hi ? u[v + m][0] : u[v + m][C - 1];
+            Fr[m] = e.circ_hi ? F[v + m][0] : F[v + m][C - 1];
+        }
+    } else {
+        rec_part<v, M>(e.l1.X1, 2, e.l1.i1, e.NT, ul, Fl);
+        rec_part<v, M>(e.r1.X1, 2, e.r1.i1, e.NT, ur, Fr);
+    }
+    V a[C + 2], f[C + 2], o[C];
+    a[0] = L::get(ul[0], ul[M - 1]);
+    f[0] = L::get(Fl[0], Fl[M - 1]);
+    a[C + 1] = L::get(ur[0], ur[M - 1]);
+    f[C + 1] = L::get(Fr[0], Fr[M - 1]);
+#pragma unroll
+    for (int k = 0; k < C; ++k) { a[k + 1] = L::get(u[v][k], u[w][k]); f[k + 1] = L::get(F[v][k], F[w][k]); }
+    if (e.nown < C) {   // the cell past a ragged end
+#pragma unroll
+        for (int k = 1; k < C; ++k) {
+            const bool here = is_cell(k, e.nown);
+            a[k + 1] = v_pick(here, a[C + 1], a[k + 1]);
+            f[k + 1] = v_pick(here, f[C + 1], f[k + 1]);
+        }
+    }
+    seg_predict<V, C, v < 4 ? RND : 0>(a, f, v_dup<V>(ic), v_dup<V>(-ic), v_dup<V>(qh), v_dup<V>(-qh), e.round4, e.round_end, o);
+#pragma unroll
+    for (int k = 0; k < C; ++k) L::put(o[k], u[v][k], u[w][k]);
+}
+
+// Corrector of variables v .. (one lane's): the new values of the own cells from u, u* and F*, stored
+// at once (held to the end they would cost 5 C registers).
+template <typename V, typename T, int C, int LIM, int v, typename Store>
+__device__ __forceinline__ void seg_correct_vars(const SegEnds& e, const T (&u)[5][C], const Store& store,
+                                                 const T (&us)[5][C], const T (&Fs)[5][C], T ics, T ffc) {
+    using L = SegLane<V, T>;
+    constexpr int M = L::N, w = v + M - 1;
+    V x[C + 4], f[C + 4], o[C], a[C];
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+        x[k + 2] = L::get(us[v][k], us[w][k]);
+        f[k + 2] = L::get(Fs[v][k], Fs[w][k]);
+    }
+    if (e.solo) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {   // cells -2, -1 and C, C + 1
+            x[j] = e.circ_lo ? x[C + j] : x[2];
+            f[j] = e.circ_lo ? f[C + j] : f[2];
+            x[C + 2 + j] = e.circ_hi ? x[2 + j] : x[C + 1];
+            f[C + 2 + j] = e.circ_hi ? f[2 + j] : f[C + 1];
+        }
+    } else {
+        T p[M], q[M];
+        rec_part<v, M>(e.l2.X2, 4, e.l2.i2, e.NT, p, q);
+        x[0] = L::get(p[0], p[M - 1]);
+        f[0] = L::get(q[0], q[M - 1]);
+        rec_part<v, M>(e.l1.X2, 4, e.l1.i2, e.NT, p, q);
+        x[1] = L::get(p[0], p[M - 1]);
+        f[1] = L::get(q[0], q[M - 1]);
+        rec_part<v, M>(e.r1.X2, 4, e.r1.i2, e.NT, p, q);
+        x[C + 2] = L::get(p[0], p[M - 1]);
+        f[C + 2] = L::get(q[0], q[M - 1]);
+        rec_part<v, M>(e.r2.X2, 4, e.r2.i2, e.NT, p, q);
+        x[C + 3] = L::get(p[0], p[M - 1]);
+        f[C + 3] = L::get(q[0], q[M - 1]);
+    }
+    if (e.nown < C) {   // the two cells past a ragged end: local cells nown and nown + 1
+#pragma unroll
+        for (int k = 1; k < C; ++k) {
+            const bool one = is_cell(k, e.nown), two = is_cell(k, e.nown + 1);
+            x[k + 2] = v_pick(one, x[C + 2], v_pick(two, x[C + 3], x[k + 2]));
+            f[k + 2] = v_pick(one, f[C + 2], v_pick(two, f[C + 3], f[k + 2]));
+        }
+        const bool next = is_cell(C - 1, e.nown);
+        x[C + 2] = v_pick(next, x[C + 3], x[C + 2]);
+        f[C + 2] = v_pick(next, f[C + 3], f[C + 2]);
+    }
+#pragma unroll
+    for (int k = 0; k < C; ++k) a[k] = L::get(u[v][k], u[w][k]);
+#pragma unroll
+    for (int j = 0; j < C + 4; ++j) x[j] = v_mul(x[j], v_splat<V>(0.5));
+    seg_correct<V, C, LIM>(a, x, f, v_dup<V>(T(0.5) * ics), v_dup<V>(T(-0.5) * ics), v_dup<V>(-ffc), e.lo_own, e.hi_own ? e.nown - 1 : C, o);
+    T p[C], q[C];
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+        if constexpr (M == 2) L::put(o[k], p[k], q[k]);
+        else p[k] = o[k];
+    }
+    store(v, p);
+    if constexpr (M == 2) store(w, q);
+}
+
+template <typename T, int C, int LIM, typename Store>
+__device__ __forceinline__ void seg_correct_all(const SegEnds& e, const T (&u)[5][C], const Store& store,
+                                                const T (&us)[5][C], const T (&Fs)[5][C], T ics, T ffc) {
+    if constexpr (sizeof(T) == 4) {
+        seg_correct_vars<F2, T, C, LIM, 0>(e, u, store, us, Fs, ics, ffc);
+        asm volatile("" ::: "memory");   // one lane's neighbours at a time: fewer live registers
+        seg_correct_vars<F2, T, C, LIM, 2>(e, u, store, us, Fs, ics, ffc);
+        asm volatile("" ::: "memory");
+        seg_correct_vars<T, T, C, LIM, 4>(e, u, store, us, Fs, ics, ffc);
+    } else {
+        seg_correct_vars<T, T, C, LIM, 0>(e, u, store, us, Fs, ics, ffc);
+        seg_correct_vars<T, T, C, LIM, 1>(e, u, store, us, Fs, ics, ffc);
+        seg_correct_vars<T, T, C, LIM, 2>(e, u, store, us, Fs, ics, ffc);
+        seg_correct_vars<T, T, C, LIM, 3>(e, u, store, us, Fs, ics, ffc);
+        seg_correct_vars<T, T, C, LIM, 4>(e, u, store, us, Fs, ics, ffc);
+    }
+}
+
+// ---- fade ends (fade_shift.m:21-45) ---------------------------------------------------------------------
+// The damping of one cell's row in a shifted array: v toward the shifted array's first value (s0, weight
+// lo), then toward its last (sN, weight hi); weights are 0 (and nothing is done) away from the ends.
 template <typename T>
-__device__ __forceinline__ T clu_max_collect(const SweepGeom& g, const T* pm, T* cm, int slot) {
-    const int lane = threadIdx.x & 31;
-    const T m = warp_max_nonneg(lane < (g.NT >> 5) ? pm[lane * 32] : T(0));
-    if (g.CL == 1) return m;
-    if (threadIdx.x == 0) cm[slot] = m;
-    cluster_sync();
-    T c = T(0);
-    if (lane < g.CL) c = cg::this_cluster().map_shared_rank(cm, lane)[slot];
-    return warp_max_nonneg(c);
+struct SegFade {
+    T lo, hi;
+    __device__ __forceinline__ T operator()(T v, T s0, T sN) const {
+        if (lo != T(0)) v = v_fma(T(1) - lo, v, lo * s0);
+        if (hi != T(0)) v = v_fma(T(1) - hi, v, hi * sN);
+        return v;
+    }
+};
+
+// Publish the last two own cells of a segment of n < C cells: the last in slot b, the one before in slot a (n >= 2;
+// a < 0: not published).  Every cell is written, those not wanted to slot 0, which the caller writes
+// afterwards: the choice is in the address, since a choice among the cells' values (by selects or by branches)
+// moves their arrays out of registers.
+template <typename T, int C>
+__device__ __forceinline__ void rec_put_tail(unsigned char* X, int slots, int a, int b, int NT, int t, const T (&u)[5][C],
+                                             const T (&F)[5][C], int n) {
+#pragma unroll
+    for (int k = C - 2; k >= 0; --k) {
+        T c[5], f[5];
+        cell(u, k, c);
+        cell(F, k, f);
+        rec_put(X, slots, is_cell(k, n - 1) ? b : (a >= 0 && is_cell(k, n - 2) ? a : 0), NT, t, c, f);
+    }
 }
 
 // VT: the artificial viscosity (VISC_*), fixed per kernel.  With viscosity each of the first two
 // stages takes one more barrier: the viscosity exchange set is published with the pencil maximum, and
-// the flux numerators (which include the viscous pressure) are published after it.
-// CLU: one pencil along x per cluster of CL CTAs (CL = 1: one CTA), placed by SegPos::init_cluster:
-// the exchanges with segments in another CTA read its shared memory through DSMEM, the barriers and the
-// pencil maxima span the cluster, and a length that C does not divide leaves the last segment ragged
-// (const ends only: its cells past the pencil's end load the end cell and, after the predictor, take the
-// end cell's half-step state, the const ghosts of every shifted array).
-template <typename T, bool MHD, int C, int VT, bool CLU = false>
+// the flux numerators (which include the viscous pressure) are published after it; every segment is whole.
+// CLU: one pencil along x per cluster of CL CTAs (CL = 1: one CTA).  FADE: a fade end on this dimension.
+template <typename T, int MHD, int C, int VT, bool CLU, bool FADE>
 __device__ __forceinline__ void fluid_seg_body(const FluidArgs& a, unsigned vblock) {
     static_assert(!CLU || VT == VISC_NONE, "cluster segments carry no viscosity");
+    static_assert(!FADE || (VT == VISC_NONE && !CLU), "fade ends: one CTA, no viscosity");
+    static_assert(C >= 2, "two cells per end are published");
     extern __shared__ __align__(16) unsigned char smem[];
-    pdl_wait();
-    // cluster launches return on `done` only, as fluid_sweep_body_general's do
-    if (a.tm->done || (a.sg.CL == 1 && a.tm->error)) return;
     __shared__ double cflp[3][MAX_WARPS];
-    __shared__ T cmax[2];
+    using U = typename SegBits<T>::U;
     const SweepGeom& g = a.sg;
-    const int NT = g.NT, S = g.G, d = g.d, d1 = g.d1, d2 = g.d2;
-    const int N = g.N;
+    const int NT = g.NT, S = g.G, d = g.d, d1 = g.d1, d2 = g.d2, N = g.N;
     const int t = threadIdx.x;
     SegPos sp;
-    if constexpr (CLU) sp.init_cluster(g, vblock);
-    else sp.init(g, vblock);
-    const int s = sp.s;
-    T* X1 = reinterpret_cast<T*>(smem);   // [20][NT]: (u, F) of the first cell, then of the last
-    T* X2 = X1 + 20 * NT;                 // [40][NT]: (u*, F*) of cells 0, 1, C-2, C-1
-    T* PM = X2 + 40 * NT;                 // [2][NT/32][32]: per-warp pencil maxima
-    double* V = reinterpret_cast<double*>(PM + 2 * (NT >> 5) * 32);   // [VISC_ROWS][NT] (viscosity only)
+    sp.init<CLU>(g, vblock);
+    const int s = sp.s, r0 = s * C;
+    const int nown = sp.colok ? (N - r0 < C ? N - r0 : C) : 0;   // own cells inside the pencil (idle threads: none)
+    unsigned char* X1 = smem;                            // (u, F) of the first and the last own cell
+    unsigned char* X2 = X1 + 2 * seg_rec_bytes<T>() * NT;   // (u*, F*) of own cells 0, 1, last - 1, last
+    U* pmax = reinterpret_cast<U*>(X2 + 4 * seg_rec_bytes<T>() * NT);   // [2][Wb] pencil maxima
+    double* V = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(pmax) + 16 * g.Wb);   // viscosity or fade anchors
+    for (int i = t; i < 2 * g.Wb; i += NT) pmax[i] = 0;
+
+    // ---- the neighbour segments --------------------------------------------------------------------
+    SegEnds e;
     const bool circ_lo = a.mode[CLS_MASS][0] == BC_CIRC, circ_hi = a.mode[CLS_MASS][1] == BC_CIRC;
+    e.circ_lo = circ_lo;
+    e.circ_hi = circ_hi;
+    e.solo = VT == VISC_NONE && !CLU && !FADE && S == 1 && N == C;   // uniform over the launch
+    e.nown = nown;
+    e.NT = NT;
+    const bool solo = e.solo;
     const int ls = d == 0 ? 1 : g.Wb;     // thread distance between consecutive segments of a pencil
     const bool lo_own = s == 0 && !circ_lo, hi_own = s == S - 1 && !circ_hi;
-    int lt = s > 0 ? t - ls : (circ_lo ? t + (S - 1) * ls : t);
-    int rt = s < S - 1 ? t + ls : (circ_hi ? t - (S - 1) * ls : t);
-    // the exchange sets holding the neighbour segments (another rank's across a cluster)
-    const T* X1l = X1;
-    const T* X1r = X1;
-    const T* X2l = X2;
-    const T* X2r = X2;
-    int nown = C;   // own cells inside the pencil (a ragged last segment: fewer; idle threads: none)
-    if constexpr (CLU) {
-        const int sc = s < S ? s : S - 1;   // idle threads read a real segment's neighbours
-        const int sl = sc > 0 ? sc - 1 : (circ_lo ? S - 1 : sc);
-        const int sr = sc < S - 1 ? sc + 1 : (circ_hi ? 0 : sc);
-        const int rl = sl / NT, rr = sr / NT;
-        lt = sl - rl * NT;
-        rt = sr - rr * NT;
-        if (rl != sp.rank) {
-            X1l = cg::this_cluster().map_shared_rank(X1, rl);
-            X2l = cg::this_cluster().map_shared_rank(X2, rl);
-        }
-        if (rr != sp.rank) {
-            X1r = cg::this_cluster().map_shared_rank(X1, rr);
-            X2r = cg::this_cluster().map_shared_rank(X2, rr);
-        }
-        nown = N - s * C < C ? N - s * C : C;
+    e.lo_own = lo_own;
+    const bool tile = sizeof(T) == 4 && a.round_cells == 0;
+    e.round4 = a.round_cells == 4;
+    e.round_end = a.round_cells && (r0 + C) % a.round_cells == 0;
+    e.hi_own = hi_own;
+    SegRef &rl1 = e.l1, &rl2 = e.l2, &rr1 = e.r1, &rr2 = e.r2;
+    int lt, rt;                  // threads of the neighbour segments (viscosity: whole segments, one CTA)
+    {
+        const int me = sp.colok ? s : (CLU ? S - 1 : 0);   // idle threads: the records of some segment
+        const int last_n = N - (S - 1) * C;                 // own cells of the last segment
+        const int sl = me > 0 ? me - 1 : (circ_lo ? S - 1 : 0);
+        const int sr = me < S - 1 ? me + 1 : (circ_hi ? 0 : S - 1);
+        const int sll = sl > 0 ? sl - 1 : (circ_lo ? S - 1 : 0);
+        const int srr = sr < S - 1 ? sr + 1 : (circ_hi ? 0 : S - 1);
+        // record of segment q: slot k1 of the first set, slot k2 of the second
+        auto ref = [&](int q, int k1, int k2) -> SegRef {
+            SegRef r;
+            int tq;
+            r.X1 = X1;
+            r.X2 = X2;
+            if constexpr (CLU) {
+                const int rk = q / NT;
+                tq = q - rk * NT;
+                if (rk != sp.rank) {
+                    r.X1 = cg::this_cluster().map_shared_rank(X1, rk);
+                    r.X2 = cg::this_cluster().map_shared_rank(X2, rk);
+                }
+            } else {
+                tq = sp.colok ? t + (q - s) * ls : t;
+            }
+            r.i1 = k1 * NT + tq;
+            r.i2 = k2 * NT + tq;
+            return r;
+        };
+        const bool lo_me = me == 0 && !circ_lo, hi_me = me == S - 1 && !circ_hi;
+        // a const end's ghosts are its end cell: slot 0 of the first segment, the last slot of the last one
+        rl1 = lo_me ? ref(me, 0, 0) : ref(sl, 1, 3);
+        rr1 = hi_me ? ref(me, 1, 3) : ref(sr, 0, 0);
+        const bool l_short = sl == S - 1 && last_n == 1, r_short = sr == S - 1 && last_n == 1;
+        rl2 = lo_me ? rl1 : (l_short ? ref(sll, 1, 3) : ref(sl, 1, 2));
+        rr2 = hi_me ? rr1 : (r_short ? (circ_hi ? ref(srr, 0, 0) : ref(sr, 1, 3)) : ref(sr, 0, 1));
+        lt = s > 0 ? t - ls : (circ_lo ? t + (S - 1) * ls : t);
+        rt = s < S - 1 ? t + ls : (circ_hi ? t - (S - 1) * ls : t);
     }
-    const double G = a.gamma;
-    const double dt = a.tm->dt;
-    const T ff = (T)(dt / a.dx);
-    const T half_ffx = (T)(0.5 * (dt / a.dx));
+
+    // ---- stage 1: load, pressure, speed, F -----------------------------------------------------------
     // vector accesses need segments on multiples of C: pencils start on one where C divides N
-    const bool vec = d == 0 && (!CLU || N % C == 0);
-    const bool ragged = CLU && nown < C;   // cells past the pencil's end: load (and later take) the end cell
-    const long long o0 = sp.base + (long long)s * C * g.sd;
+    const bool vec = d == 0 && N % C == 0;
+    const int sd = (int)g.sd;
+    const int o0 = sp.base + r0 * sd;
     // momentum and cell-centred B in sweep-rotated order: component 0 along the sweep, then d1, d2
-    void* qv[5] = {a.q[Q_RHO], a.q[Q_PX + d], a.q[Q_PX + d1], a.q[Q_PX + d2], a.q[Q_E]};
+    void* const qv[5] = {a.q[Q_RHO], a.q[Q_PX + d], a.q[Q_PX + d1], a.q[Q_PX + d2], a.q[Q_E]};
+    void* const bv[3] = {a.q[Q_CBX + d], a.q[Q_CBX + d1], a.q[Q_CBX + d2]};
     const bool ub[3] = {a.use_b[d] != 0, a.use_b[d1] != 0, a.use_b[d2] != 0};
     // rotated slots of the natural x, y, z components (the CSW sound speed sums in natural order)
     const int nx = d == 0 ? 0 : (d1 == 0 ? 1 : 2), ny = d == 1 ? 0 : (d1 == 1 ? 1 : 2), nz = d == 2 ? 0 : (d1 == 2 ? 1 : 2);
     constexpr bool LOADB = MHD || VT == VISC_CSW;   // cswSoundSpeed reads every cell-centred component
-
-    // ---- stage 1: load, pressure, speed, F -------------------------------------------------------
+    pdl_wait();
+    const int stop = a.tm->done | (!CLU || g.CL == 1 ? a.tm->error : 0);   // cluster launches return on `done` only
+    const double dt = a.tm->dt, dq = dt * a.inv_dx, dtx = fma(fma(-dq, a.dx, dt), a.inv_dx, dq);   // dt / dx, one residual step
     T u[5][C], bb[3][C], F[5][C];
-    // sum of squares of the cell-centred B components without isZero, in rotated order (recomputed
-    // where needed instead of kept: it would hold 2C registers for the whole kernel)
-    auto bsq = [&](const T (&b)[3][C], int k) {
-        double m = 0.0;
+    auto load_u = [&](int v, T (&w)[C]) { win_load<T, C, true>(qv[v], o0, sd, vec, nown, v == 0 ? T(1) : T(0), w); };
+    auto load_b = [&]() {   // the cell-centred B, which a fluid sweep leaves alone
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-            if (MHD && ub[c]) m = m + (double)b[c][k] * (double)b[c][k];
-        return m;
+        for (int c = 0; c < 3; ++c) {
+            if (LOADB) win_load<T, C, true>(bv[c], o0, sd, vec, nown, T(0), bb[c]);
+            else
+#pragma unroll
+                for (int k = 0; k < C; ++k) bb[c][k] = T(0);
+        }
     };
-    if (sp.colok && ragged) {
+#pragma unroll
+    for (int v = 0; v < 5; ++v) load_u(v, u[v]);
+    load_b();
+    SegFade<T> fw[C];
+    const bool fade_lo = FADE && a.mode[CLS_MASS][0] == BC_FADE, fade_hi = FADE && a.mode[CLS_MASS][1] == BC_FADE;
+    if constexpr (FADE) {
+        const int f = a.fade_f;
 #pragma unroll
         for (int k = 0; k < C; ++k) {
-            const long long o = sp.base + (long long)(k < nown ? s * C + k : N - 1) * g.sd;
-#pragma unroll
-            for (int v = 0; v < 5; ++v) u[v][k] = ldq<T>(qv[v], o);
-            if (LOADB) {
-                bb[0][k] = ldq<T>(a.q[Q_CBX + d], o);
-                bb[1][k] = ldq<T>(a.q[Q_CBX + d1], o);
-                bb[2][k] = ldq<T>(a.q[Q_CBX + d2], o);
-            } else {
-                bb[0][k] = bb[1][k] = bb[2][k] = T(0);
-            }
-        }
-    } else if (sp.colok) {
-#pragma unroll
-        for (int v = 0; v < 5; ++v) seg_load<T, C>(qv[v], o0, g.sd, vec, u[v]);
-        if (LOADB) {
-            seg_load<T, C>(a.q[Q_CBX + d], o0, g.sd, vec, bb[0]);
-            seg_load<T, C>(a.q[Q_CBX + d1], o0, g.sd, vec, bb[1]);
-            seg_load<T, C>(a.q[Q_CBX + d2], o0, g.sd, vec, bb[2]);
-        } else {
-#pragma unroll
-            for (int k = 0; k < C; ++k) bb[0][k] = bb[1][k] = bb[2][k] = T(0);
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < C; ++k) {
-            u[0][k] = T(1);
-            u[1][k] = u[2][k] = u[3][k] = u[4][k] = T(0);
-            bb[0][k] = bb[1][k] = bb[2][k] = T(0);
+            const int r = r0 + k;
+            fw[k].lo = k < nown && r < f ? (T)a.fade[r] : T(0);
+            fw[k].hi = k < nown && r >= N - f ? (T)a.fade[N - 1 - r] : T(0);
         }
     }
-    T lmax = T(0);
-    T cf;
+    if (stop) return;   // after the loads are on their way: the flags take as long as they do
+    __syncthreads();    // the maxima are zeroed
+    T u0[5][C];   // the variables before the sweep
+#pragma unroll
+    for (int v = 0; v < 5; ++v)
+#pragma unroll
+        for (int k = 0; k < C; ++k) u0[v][k] = u[v][k];
+    const SegPressure pk(a.gamma);
+    // sum of squares of the cell-centred B components without isZero
+    auto bsq = [&](int k) {
+        double m = 0.0;
+        if constexpr (MHD)
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                if (ub[c]) m = fma((double)bb[c][k], (double)bb[c][k], m);
+        return m;
+    };
+    const bool whole = nown == C;
+    auto put1 = [&](const T (&w)[5][C], const T (&Fw)[5][C]) {
+        if (solo) return;
+        T c[5], f[5];
+        if (!whole) {
+            rec_put_tail(X1, 2, -1, 1, NT, t, w, Fw, nown);
+        } else {
+            cell(w, C - 1, c);
+            cell(Fw, C - 1, f);
+            rec_put(X1, 2, 1, NT, t, c, f);
+        }
+        cell(w, 0, c);
+        cell(Fw, 0, f);
+        rec_put(X1, 2, 0, NT, t, c, f);
+    };
+    // fade: (w, F) of the pencil's rows 0, 1, N-2, N-1 as anchor records of stage st
+    T* AN = reinterpret_cast<T*>(V);
+    const int ab = sp.b < g.Wb ? sp.b : 0;   // idle threads past the pencils read pencil 0's
+    const bool near_end = r0 < 2 || r0 + C > N - 2;
+    auto row_slot = [&](int r) { return r == 0 ? 0 : (r == 1 ? 1 : (r == N - 2 ? 2 : (r == N - 1 ? 3 : -1))); };
+    auto put_anchors = [&](int st, const T (&w)[5][C], const T (&Fw)[5][C]) {
+        if (!near_end) return;
+#pragma unroll
+        for (int k = 0; k < C; ++k) {
+            const int q = k < nown ? row_slot(r0 + k) : -1;
+            if (q >= 0) {
+                T* p = AN + ((st * 4 + q) * g.Wb + sp.b) * 10;
+#pragma unroll
+                for (int v = 0; v < 5; ++v) { p[v] = w[v][k]; p[5 + v] = Fw[v][k]; }
+            }
+        }
+    };
+    T lmax = T(0), cf;
     if constexpr (VT == VISC_NONE) {
 #pragma unroll
         for (int k = 0; k < C; ++k) {
-            const double m = bsq(bb, k);
-            const T uu[5] = {u[0][k], u[1][k], u[2][k], u[3][k], u[4][k]};
+            T c[5], Fk[5], p, cs, ir;
+            cell(u, k, c);
             const T b3[3] = {bb[0][k], bb[1][k], bb[2][k]};
-            T p;
-            const T spd = press_speed_rot<T>(G, uu, m, p);
-            if (sp.colok) lmax = fmax(lmax, spd);
-            T Fk[5];
-            flux_num_rot<T>(uu, b3, p, Fk);
+            const T spd = seg_pressure<MHD>(pk, c, bsq(k), p, cs, ir);
+            if (k < nown) lmax = fmax(lmax, spd);
+            seg_flux<T, MHD>(d, tile, c, b3, p, ir, Fk);
 #pragma unroll
             for (int v = 0; v < 5; ++v) F[v][k] = Fk[v];
         }
-#pragma unroll
-        for (int v = 0; v < 5; ++v) {
-            X1[v * NT + t] = u[v][0];
-            X1[(5 + v) * NT + t] = F[v][0];
-            X1[(10 + v) * NT + t] = u[v][C - 1];
-            X1[(15 + v) * NT + t] = F[v][C - 1];
-        }
-        if constexpr (CLU) {
-            clu_max_publish(lmax, PM);
-            sp_sync<CLU>(g);
-            cf = clu_max_collect(g, PM, cmax, 0);   // freezing speed (wFluidFlux.m:18-22)
-        } else {
-            const T wv1 = seg_max_publish(g, lmax, PM);
-            __syncthreads();
-            cf = seg_max_collect(g, sp.b, wv1, PM);   // freezing speed (wFluidFlux.m:18-22)
-        }
+        put1(u, F);
+        if constexpr (FADE) put_anchors(0, u, F);
+        seg_max_publish<T, CLU>(g, sp, lmax, pmax);
+        if (!solo) sp_sync<CLU>(g);
+        cf = seg_max_collect<T, CLU>(g, sp, lmax, pmax);   // freezing speed (wFluidFlux.m:18-22)
     } else {
-        T P[C], CS[C];
+        T P[C], CS[C], IR[C];
         double vel[C], snd[C], q[C];
 #pragma unroll
         for (int k = 0; k < C; ++k) {
-            const double m = bsq(bb, k);
-            const T uu[5] = {u[0][k], u[1][k], u[2][k], u[3][k], u[4][k]};
-            const T spd = press_speed_rot<T>(G, uu, m, P[k], CS[k]);
-            if (sp.colok) lmax = fmax(lmax, spd);
+            T c[5];
+            cell(u, k, c);
+            const T spd = seg_pressure<MHD>(pk, c, bsq(k), P[k], CS[k], IR[k]);
+            if (k < nown) lmax = fmax(lmax, spd);
         }
-        seg_visc_publish<T, C, VT>(u, bb, G, nx, ny, nz, V, NT, t, vel, snd);
-        const T wv1 = seg_max_publish(g, lmax, PM);
+        seg_visc_publish<T, C, VT>(u, bb, a.gamma, nx, ny, nz, V, NT, t, vel, snd);
+        seg_max_publish<T, CLU>(g, sp, lmax, pmax);
         __syncthreads();
-        cf = seg_max_collect(g, sp.b, wv1, PM);   // freezing speed (wFluidFlux.m:18-22), before the viscosity
-        seg_visc_terms<T, C, VT>(a, G, u, CS, vel, snd, V, NT, lt, rt, lo_own, hi_own, q);
+        cf = seg_max_collect<T, CLU>(g, sp, lmax, pmax);   // freezing speed (wFluidFlux.m:18-22), before the viscosity
+        seg_visc_terms<T, C, VT>(a, a.gamma, u, CS, vel, snd, V, NT, lt, rt, lo_own, hi_own, q);
 #pragma unroll
         for (int k = 0; k < C; ++k) {
-            const T uu[5] = {u[0][k], u[1][k], u[2][k], u[3][k], u[4][k]};
-            const T b3[3] = {MHD ? bb[0][k] : T(0), MHD ? bb[1][k] : T(0), MHD ? bb[2][k] : T(0)};
-            T Fk[5];
-            flux_num_rot<T>(uu, b3, visc_add<T>(P[k], q[k]), Fk);   // press + viscosity.solve (wFluidFlux.m:24)
+            T c[5], Fk[5];
+            cell(u, k, c);
+            const T b3[3] = {bb[0][k], bb[1][k], bb[2][k]};
+            seg_flux<T, MHD>(d, tile, c, b3, visc_add<T>(P[k], q[k]), IR[k], Fk);   // press + viscosity.solve (wFluidFlux.m:24)
 #pragma unroll
             for (int v = 0; v < 5; ++v) F[v][k] = Fk[v];
         }
-#pragma unroll
-        for (int v = 0; v < 5; ++v) {
-            X1[v * NT + t] = u[v][0];
-            X1[(5 + v) * NT + t] = F[v][0];
-            X1[(10 + v) * NT + t] = u[v][C - 1];
-            X1[(15 + v) * NT + t] = F[v][C - 1];
-        }
+        put1(u, F);
         __syncthreads();
     }
-    T ic;
-    if constexpr (sizeof(T) == 4) ic = __frcp_rn(cf);
-    else ic = T(1) / cf;
 
     // ---- stage 2: predictor (relaxingFluid.m:30-39) and the half-step pressure, speed, F ----------
-    T us[5][C], Fs[5][C];
-    const T hfc = half_ffx * cf;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-        // R = (u + F/c_f)/2 at cells -1 .. C-1 (index j + 1), L = (u - F/c_f)/2 at cells 0 .. C (index j)
-        T R[C + 1], L[C + 1];
-#pragma unroll
-        for (int k = 0; k < C; ++k) {
-            const T w = F[v][k] * ic;
-            R[k + 1] = T(0.5) * (u[v][k] + w);
-            L[k] = T(0.5) * (u[v][k] - w);
-        }
-        R[0] = lo_own ? R[1] : T(0.5) * (X1l[(10 + v) * NT + lt] + X1l[(15 + v) * NT + lt] * ic);
-        L[C] = hi_own ? L[C - 1] : T(0.5) * (X1r[v * NT + rt] - X1r[(5 + v) * NT + rt] * ic);
-#pragma unroll
-        for (int k = 0; k < C; ++k) us[v][k] = u[v][k] - hfc * (R[k + 1] - R[k] + L[k] - L[k + 1]);
-        if (ragged && nown > 0) {   // cells past the end take the end cell's half-step state
-            T e = us[v][0];
-#pragma unroll
-            for (int k = 1; k < C; ++k)
-                if (k == nown - 1) e = us[v][k];
-#pragma unroll
-            for (int k = 1; k < C; ++k)
-                if (k >= nown) us[v][k] = e;
-        }
-    }
-    T lmax2 = T(0);
-    T P2[C], CS2[C];
-#pragma unroll
-    for (int k = 0; k < C; ++k) {
-        us[0][k] = us[0][k] > (T)a.minmass ? us[0][k] : (T)a.minmass;   // max(rho, MINMASS), NaN -> MINMASS
-        if (!sp.colok) { us[0][k] = T(1); us[1][k] = us[2][k] = us[3][k] = us[4][k] = T(0); }
-        const T uu[5] = {us[0][k], us[1][k], us[2][k], us[3][k], us[4][k]};
-        if constexpr (VT == VISC_NONE) {
-            const T b3[3] = {bb[0][k], bb[1][k], bb[2][k]};
-            T p2;
-            const T spd = press_speed_rot<T>(G, uu, bsq(bb, k), p2);   // relaxingFluid.m:47-50
-            if (sp.colok) lmax2 = fmax(lmax2, spd);
-            T Fk[5];
-            flux_num_rot<T>(uu, b3, p2, Fk);
-#pragma unroll
-            for (int v = 0; v < 5; ++v) Fs[v][k] = Fk[v];
+    T ic;
+    if constexpr (sizeof(T) == 4) ic = __frcp_rn(cf);
+    else ic = recip(cf);
+    const T hfc = (T)(0.5 * dtx) * cf;
+    if constexpr (!FADE) {
+        const T qh = T(0.5) * hfc;
+        constexpr int RND = seg_round_mode<T, MHD, C>();
+        if constexpr (sizeof(T) == 4) {
+            seg_predict_vars<F2, T, C, RND, 0>(e, u, F, ic, qh);
+            asm volatile("" ::: "memory");   // one lane's neighbours at a time: fewer live registers
+            seg_predict_vars<F2, T, C, RND, 2>(e, u, F, ic, qh);
+            asm volatile("" ::: "memory");
+            seg_predict_vars<T, T, C, RND, 4>(e, u, F, ic, qh);
         } else {
-            const T spd = press_speed_rot<T>(G, uu, bsq(bb, k), P2[k], CS2[k]);
-            if (sp.colok) lmax2 = fmax(lmax2, spd);
+            seg_predict_vars<T, T, C, RND, 0>(e, u, F, ic, qh);
+            seg_predict_vars<T, T, C, RND, 1>(e, u, F, ic, qh);
+            seg_predict_vars<T, T, C, RND, 2>(e, u, F, ic, qh);
+            seg_predict_vars<T, T, C, RND, 3>(e, u, F, ic, qh);
+            seg_predict_vars<T, T, C, RND, 4>(e, u, F, ic, qh);
+        }
+    } else {
+        T ul[5], Fl[5], ur[5], Fr[5];
+        rec_get(rl1.X1, 2, rl1.i1, NT, ul, Fl);
+        rec_get(rr1.X1, 2, rr1.i1, NT, ur, Fr);
+        const T* an = AN + ab * 10;
+        const int ar = 10 * g.Wb;   // between anchor rows
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            T R[C + 1], L[C + 1];   // R at cells -1 .. C-1 (j + 1), L at cells 0 .. C (j)
+            R[0] = T(0.5) * v_fma(Fl[v], ic, ul[v]);
+            L[C] = T(0.5) * v_fma(Fr[v], -ic, ur[v]);
+#pragma unroll
+            for (int k = 0; k < C; ++k) {
+                R[k + 1] = T(0.5) * v_fma(F[v][k], ic, u[v][k]);
+                L[k] = T(0.5) * v_fma(F[v][k], -ic, u[v][k]);
+            }
+            const T Le = L[C];   // past a ragged end
+#pragma unroll
+            for (int k = 1; k < C; ++k) L[k] = v_pick(is_cell(k, nown), Le, L[k]);
+            const T R0 = T(0.5) * v_fma(an[5 + v], ic, an[v]), RN = T(0.5) * v_fma(an[2 * ar + 5 + v], ic, an[2 * ar + v]);
+            const T L0 = T(0.5) * v_fma(an[ar + 5 + v], -ic, an[ar + v]), LN = T(0.5) * v_fma(an[3 * ar + 5 + v], -ic, an[3 * ar + v]);
+#pragma unroll
+            for (int k = 0; k < C; ++k) {
+                const T Rm = fade_lo ? fw[k](R[k], R0, RN) : R[k], Lp = fade_hi ? fw[k](L[k + 1], L0, LN) : L[k + 1];
+                u[v][k] = v_fma(-hfc, R[k + 1] - Rm + L[k] - Lp, u[v][k]);
+            }
         }
     }
-    if constexpr (VT != VISC_NONE) {
-        // the viscosity of the half-step state: one more barrier before its fluxes are published
-        double vel[C], snd[C], q[C];
-        seg_visc_publish<T, C, VT>(us, bb, G, nx, ny, nz, V, NT, t, vel, snd);
-        const T wv2 = seg_max_publish(g, lmax2, PM + (NT >> 5) * 32);
-        __syncthreads();
-        lmax2 = seg_max_collect(g, sp.b, wv2, PM + (NT >> 5) * 32);
-        seg_visc_terms<T, C, VT>(a, G, us, CS2, vel, snd, V, NT, lt, rt, lo_own, hi_own, q);
+    T (&us)[5][C] = u, Fs[5][C];   // the half-step state in u's place
+    T lmax2 = T(0), cfs;
+    const T mm = (T)a.minmass;
+    {
+        T P2[C], CS2[C], IR2[C];
 #pragma unroll
         for (int k = 0; k < C; ++k) {
-            const T uu[5] = {us[0][k], us[1][k], us[2][k], us[3][k], us[4][k]};
-            const T b3[3] = {MHD ? bb[0][k] : T(0), MHD ? bb[1][k] : T(0), MHD ? bb[2][k] : T(0)};
-            T Fk[5];
-            flux_num_rot<T>(uu, b3, visc_add<T>(P2[k], q[k]), Fk);
+            us[0][k] = us[0][k] > mm ? us[0][k] : mm;   // max(rho, MINMASS), NaN -> MINMASS
+            if (k >= nown) { us[0][k] = T(1); us[1][k] = us[2][k] = us[3][k] = us[4][k] = T(0); }
+            T c[5], Fk[5];
+            cell(us, k, c);
+            const T spd = seg_pressure<MHD>(pk, c, bsq(k), P2[k], CS2[k], IR2[k]);   // relaxingFluid.m:47-50
+            if (k < nown) lmax2 = fmax(lmax2, spd);
+            if constexpr (VT == VISC_NONE) {
+                const T b3[3] = {bb[0][k], bb[1][k], bb[2][k]};
+                seg_flux<T, MHD>(d, tile, c, b3, P2[k], IR2[k], Fk);
 #pragma unroll
-            for (int v = 0; v < 5; ++v) Fs[v][k] = Fk[v];
+                for (int v = 0; v < 5; ++v) Fs[v][k] = Fk[v];
+            }
+        }
+        if constexpr (VT != VISC_NONE) {
+            // the viscosity of the half-step state: one more barrier before its fluxes are published
+            double vel[C], snd[C], q[C];
+            seg_visc_publish<T, C, VT>(us, bb, a.gamma, nx, ny, nz, V, NT, t, vel, snd);
+            seg_max_publish<T, CLU>(g, sp, lmax2, pmax + g.Wb);
+            __syncthreads();
+            seg_visc_terms<T, C, VT>(a, a.gamma, us, CS2, vel, snd, V, NT, lt, rt, lo_own, hi_own, q);
+#pragma unroll
+            for (int k = 0; k < C; ++k) {
+                T c[5], Fk[5];
+                cell(us, k, c);
+                const T b3[3] = {bb[0][k], bb[1][k], bb[2][k]};
+                seg_flux<T, MHD>(d, tile, c, b3, visc_add<T>(P2[k], q[k]), IR2[k], Fk);
+#pragma unroll
+                for (int v = 0; v < 5; ++v) Fs[v][k] = Fk[v];
+            }
         }
     }
-    const int c1 = C > 1 ? 1 : 0;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-        X2[v * NT + t] = us[v][0];
-        X2[(5 + v) * NT + t] = Fs[v][0];
-        X2[(10 + v) * NT + t] = us[v][c1];
-        X2[(15 + v) * NT + t] = Fs[v][c1];
-        X2[(20 + v) * NT + t] = us[v][C - 1 - c1];
-        X2[(25 + v) * NT + t] = Fs[v][C - 1 - c1];
-        X2[(30 + v) * NT + t] = us[v][C - 1];
-        X2[(35 + v) * NT + t] = Fs[v][C - 1];
+    if (!solo) {
+        T c[5], f[5];
+        if (!whole) {
+            rec_put_tail(X2, 4, 2, 3, NT, t, us, Fs, nown);
+        } else {
+            cell(us, C - 2, c);
+            cell(Fs, C - 2, f);
+            rec_put(X2, 4, 2, NT, t, c, f);
+            cell(us, C - 1, c);
+            cell(Fs, C - 1, f);
+            rec_put(X2, 4, 3, NT, t, c, f);
+        }
+        cell(us, 0, c);
+        cell(Fs, 0, f);
+        rec_put(X2, 4, 0, NT, t, c, f);
+        cell(us, 1, c);
+        cell(Fs, 1, f);
+        rec_put(X2, 4, 1, NT, t, c, f);
     }
-    T cfs;   // freezing speed of the half step
-    if constexpr (CLU) {
-        clu_max_publish(lmax2, PM + (NT >> 5) * 32);
-        sp_sync<CLU>(g);
-        cfs = clu_max_collect(g, PM + (NT >> 5) * 32, cmax, 1);
-    } else if constexpr (VT == VISC_NONE) {
-        const T wv2 = seg_max_publish(g, lmax2, PM + (NT >> 5) * 32);
-        __syncthreads();
-        cfs = seg_max_collect(g, sp.b, wv2, PM + (NT >> 5) * 32);
-    } else {
-        __syncthreads();
-        cfs = lmax2;
-    }
+    if constexpr (FADE) put_anchors(1, us, Fs);
+    if constexpr (VT == VISC_NONE) seg_max_publish<T, CLU>(g, sp, lmax2, pmax + g.Wb);
+    if (!solo) sp_sync<CLU>(g);
+    cfs = seg_max_collect<T, CLU>(g, sp, lmax2, pmax + g.Wb);   // freezing speed of the half step
     T ics;
     if constexpr (sizeof(T) == 4) ics = __frcp_rn(cfs);
-    else ics = T(1) / cfs;
+    else ics = recip(cfs);
 
     pdl_trigger();
     // ---- stage 3: corrector fluxes, TVD limiter, update (relaxingFluid.m:52-71) -------------------
-    T unew[5][C];
-    const T ffc = ff * cfs;
+    // each variable is stored as soon as it is updated: nobody else reads this thread's cells
+    const T mo = (T)a.minmass_out;
+    auto store_u = [&](int v, T (&w)[C]) {
+        if (v == 0)
 #pragma unroll
-    for (int v = 0; v < 5; ++v) {
-        const T* Xl = X2l + v * NT;
-        const T* Xr = X2r + v * NT;
-        const int nc = CLU ? nown : C;
-        if (a.limiter == LIM_VANLEER)
-            seg_correct<T, C, LIM_VANLEER>(u[v], us[v], Fs[v], Xl, Xr, NT, lt, rt, lo_own, hi_own, ics, ffc, unew[v], nc);
-        else if (a.limiter == LIM_SUPERBEE)
-            seg_correct<T, C, LIM_SUPERBEE>(u[v], us[v], Fs[v], Xl, Xr, NT, lt, rt, lo_own, hi_own, ics, ffc, unew[v], nc);
-        else
-            seg_correct<T, C, LIM_MINMOD>(u[v], us[v], Fs[v], Xl, Xr, NT, lt, rt, lo_own, hi_own, ics, ffc, unew[v], nc);
+            for (int k = 0; k < C; ++k) w[k] = w[k] > mo ? w[k] : mo;
+        win_store<T, C>(qv[v], o0, sd, vec, nown, w);
+    };
+    const T ffc = (T)dtx * cfs;
+    if constexpr (!FADE) {
+        if (a.limiter == LIM_VANLEER) seg_correct_all<T, C, LIM_VANLEER>(e, u0, store_u, us, Fs, ics, ffc);
+        else if (a.limiter == LIM_SUPERBEE) seg_correct_all<T, C, LIM_SUPERBEE>(e, u0, store_u, us, Fs, ics, ffc);
+        else seg_correct_all<T, C, LIM_MINMOD>(e, u0, store_u, us, Fs, ics, ffc);
+    } else {
+        T hl[5], hFl[5], hr[5], hFr[5];   // cell -1 and the one past the last own cell
+        rec_get(rl1.X2, 4, rl1.i2, NT, hl, hFl);
+        rec_get(rr1.X2, 4, rr1.i2, NT, hr, hFr);
+        const T* an = AN + (4 * g.Wb + ab) * 10;
+        const int ar = 10 * g.Wb;
+        T Rl[5][C], Ll[5][C], e1[5], e2[5];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            T R[C + 2], L[C + 2];   // cells -1 .. C (j + 1)
+#pragma unroll
+            for (int j = -1; j <= C; ++j) {
+                const bool past = j > 0 && j < C && is_cell(j, nown);   // past a ragged end
+                const T x = j < 0 ? hl[v] : (j < C ? v_pick(past, hr[v], us[v][j < C && j >= 0 ? j : 0]) : hr[v]);
+                const T f = j < 0 ? hFl[v] : (j < C ? v_pick(past, hFr[v], Fs[v][j < C && j >= 0 ? j : 0]) : hFr[v]);
+                R[j + 1] = T(0.5) * v_fma(f, ics, x);
+                L[j + 1] = T(0.5) * v_fma(f, -ics, x);
+            }
+            T aR[4], aL[4];   // rows 0, 1, N-2, N-1
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const T x = an[q * ar + v], f = an[q * ar + 5 + v];
+                aR[q] = T(0.5) * v_fma(f, ics, x);
+                aL[q] = T(0.5) * v_fma(f, -ics, x);
+            }
+#pragma unroll
+            for (int k = 0; k < C; ++k) {
+                const T r = R[k + 1], l = L[k + 1];
+                const T Rm = fade_lo ? fw[k](R[k], aR[0], aR[2]) : R[k], Rp = fade_hi ? fw[k](R[k + 2], aR[1], aR[3]) : R[k + 2];
+                const T Lm = fade_lo ? fw[k](L[k], aL[0], aL[2]) : L[k], Lp = fade_hi ? fw[k](L[k + 2], aL[1], aL[3]) : L[k + 2];
+                T cr, cl;
+                if (a.limiter == LIM_VANLEER) { cr = v_limit<LIM_VANLEER>(r - Rm, Rp - r); cl = v_limit<LIM_VANLEER>(Lm - l, l - Lp); }
+                else if (a.limiter == LIM_SUPERBEE) { cr = v_limit<LIM_SUPERBEE>(r - Rm, Rp - r); cl = v_limit<LIM_SUPERBEE>(Lm - l, l - Lp); }
+                else { cr = v_limit<LIM_MINMOD>(r - Rm, Rp - r); cl = v_limit<LIM_MINMOD>(Lm - l, l - Lp); }
+                Rl[v][k] = r + cr;
+                Ll[v][k] = l + cl;
+            }
+        }
+        // the limited fluxes next to the segment and at the anchor rows (the first exchange set is free again)
+        if (!whole) {
+            rec_put_tail(X1, 2, -1, 1, NT, t, Rl, Ll, nown);
+        } else {
+            cell(Rl, C - 1, e1);
+            cell(Ll, C - 1, e2);
+            rec_put(X1, 2, 1, NT, t, e1, e2);
+        }
+        cell(Rl, 0, e1);
+        cell(Ll, 0, e2);
+        rec_put(X1, 2, 0, NT, t, e1, e2);
+        T* lf = AN + 80 * g.Wb;   // [4][Wb][5]: Rl at rows 0 and N-2, Ll at rows 1 and N-1
+        if (near_end) {
+#pragma unroll
+            for (int k = 0; k < C; ++k) {
+                const int q = k < nown ? row_slot(r0 + k) : -1;
+                if (q >= 0)
+#pragma unroll
+                    for (int v = 0; v < 5; ++v) lf[(q * g.Wb + sp.b) * 5 + v] = (q & 1) ? Ll[v][k] : Rl[v][k];
+            }
+        }
+        __syncthreads();
+        T Rn[5], Ln[5], x[5];   // Rl of cell -1, Ll past the last own cell
+        rec_get(X1, 2, rl1.i1, NT, Rn, x);   // slot 1 of the left neighbour (a const end's is not used)
+        rec_get(X1, 2, rr1.i1, NT, x, Ln);   // slot 0 of the right one
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            const int fr = 5 * g.Wb;
+            T un[C];
+            const T R0 = lf[ab * 5 + v], L0 = lf[fr + ab * 5 + v], RN = lf[2 * fr + ab * 5 + v], LN = lf[3 * fr + ab * 5 + v];
+#pragma unroll
+            for (int k = 0; k < C; ++k) {
+                T Rm = k > 0 ? Rl[v][k > 0 ? k - 1 : 0] : (lo_own ? Rl[v][0] : Rn[v]);
+                T Lp = k < C - 1 ? Ll[v][k < C - 1 ? k + 1 : 0] : Ln[v];
+                if (k == nown - 1) Lp = hi_own ? Ll[v][k] : Ln[v];
+                if (fade_lo) Rm = fw[k](Rm, R0, RN);
+                if (fade_hi) Lp = fw[k](Lp, L0, LN);
+                un[k] = v_fma(-ffc, Rl[v][k] - Rm + Ll[v][k] - Lp, u0[v][k]);
+            }
+            store_u(v, un);
+        }
     }
     // the other ranks have read this CTA's exchange sets before it moves on (and may exit)
     if (CLU && g.CL > 1) cluster_sync();
-    double m3[3] = {0.0, 0.0, 0.0};   // rotated order
-    bool bad = false;
-    T cb[3][C];   // the CFL pass reloads the cell-centred B (cache hits; one sweep in six)
-    if (a.cfl && sp.colok && MHD && ragged) {
+    if (a.cfl) {   // fused CFL maxima of the new state, read back (TimeManager.m:65-77)
+        double m3[3] = {0.0, 0.0, 0.0};   // rotated order
+        bool bad = false;
 #pragma unroll
-        for (int k = 0; k < C; ++k) {
-            const long long o = sp.base + (long long)(k < nown ? s * C + k : N - 1) * g.sd;
-            cb[0][k] = ldq<T>(a.q[Q_CBX + d], o);
-            cb[1][k] = ldq<T>(a.q[Q_CBX + d1], o);
-            cb[2][k] = ldq<T>(a.q[Q_CBX + d2], o);
-        }
-    } else if (a.cfl && sp.colok && MHD) {
-        seg_load<T, C>(a.q[Q_CBX + d], o0, g.sd, vec, cb[0]);
-        seg_load<T, C>(a.q[Q_CBX + d1], o0, g.sd, vec, cb[1]);
-        seg_load<T, C>(a.q[Q_CBX + d2], o0, g.sd, vec, cb[2]);
-    }
-#pragma unroll
-    for (int k = 0; k < C; ++k) {
-        unew[0][k] = unew[0][k] > (T)a.minmass_out ? unew[0][k] : (T)a.minmass_out;
-        if (a.cfl && sp.colok && k < nown) {   // fused CFL maxima of the new state (TimeManager.m:65-77)
-            double sp3[3];
-            cfl_speeds(G, (double)unew[0][k], (double)unew[1][k], (double)unew[2][k], (double)unew[3][k],
-                       (double)unew[4][k], MHD ? bsq(cb, k) : 0.0, sp3);
-            bad = bad || !isfinite(sp3[0] + sp3[1] + sp3[2]);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) m3[c] = fmax(m3[c], sp3[c]);
-        }
-    }
-    if (sp.colok && ragged) {
+        for (int v = 0; v < 5; ++v) load_u(v, u[v]);
 #pragma unroll
         for (int k = 0; k < C; ++k)
-            if (k < nown)
+            if (k < nown) {
+                double sp3[3];
+                cfl_speeds(a.gamma, (double)u[0][k], (double)u[1][k], (double)u[2][k], (double)u[3][k], (double)u[4][k], bsq(k), sp3);
+                bad = bad || !isfinite(sp3[0] + sp3[1] + sp3[2]);
 #pragma unroll
-                for (int v = 0; v < 5; ++v) stq<T>(qv[v], o0 + (long long)k * g.sd, unew[v][k]);
-    } else if (sp.colok) {
-#pragma unroll
-        for (int v = 0; v < 5; ++v) seg_store<T, C>(qv[v], o0, g.sd, vec, unew[v]);
-    }
-    if (a.cfl) {
+                for (int c = 0; c < 3; ++c) m3[c] = fmax(m3[c], sp3[c]);
+            }
         if (a.cfl & CFL_CHECK_NONFINITE) flag_nonfinite(a.tm, bad);
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -771,35 +1170,28 @@ __device__ __forceinline__ void fluid_seg_body(const FluidArgs& a, unsigned vblo
     }
 }
 
-template <typename T, bool MHD, int C, int VT = VISC_NONE>
-__global__ void __launch_bounds__(512, 1) fluid_seg_kernel(const __grid_constant__ FluidArgs a) {
-    fluid_seg_body<T, MHD, C, VT>(a, blockIdx.x);
+// What bounds it (256^3 mixed, x, 351 us now): warp issue -- the FP64 pressure recovery, the limiters and the
+// fluxes -- beside HBM, whose 872 MB need 131 us at 6.65 TB/s; y and z (532 and 557 us) also wait for their strided rows of
+// 32 bytes.  The tiling that came before (one FP32 lane per instruction, whole-CTA barriers around idle threads, R and
+// L kept apart) took 408, 583 and 584 us; FP64 pencils and fade ends ran on the pencil tiles (96^3 FP64: 72, 112 and
+// 106 us against 51, 61 and 61 us; 96^3 hydrodynamic fade: 77, 103 and 103 us against 49, 51 and 51 us).  At 128 registers 16 warps share an SM; 80
+// registers for 24 warps spill more than they hide (256^3 y 649 -> 704 us), and persistent CTAs that fetch the
+// next bundle with cp.async lose to plain loads (x 345 -> 410 us, y 593 -> 1020 us: 4-byte copies of strided rows).
+// FP64 kernels of 3 and 4 cells a thread take CTAs of at most 256 threads with all 255 registers a thread can
+// have (MAXT): at 128 they spill.  The others run at 128, 16 warps an SM.
+template <typename T, int MHD, int C, int VT, bool CLU, bool FADE, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1) fluid_seg_kernel(const __grid_constant__ FluidArgs a) {
+    fluid_seg_body<T, MHD, C, VT, CLU, FADE>(a, blockIdx.x);
 }
 
-template <typename T, bool MHD, int C>
-__global__ void __launch_bounds__(512, 1) fluid_seg_batch_kernel(const FluidArgs* __restrict__ args,
+template <typename T, int MHD, int C, bool CLU, bool FADE, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1) fluid_seg_batch_kernel(const FluidArgs* __restrict__ args,
                                                                   const BlockMap* __restrict__ map) {
     __shared__ FluidArgs sa;
     const BlockMap bm = map[blockIdx.x];
     load_member_args(sa, args + bm.member);
     __syncthreads();
-    fluid_seg_body<T, MHD, C, VISC_NONE>(sa, (unsigned)bm.block);
-}
-
-// One pencil along x per cluster of CTAs, or per CTA with a ragged last segment (fluid_seg_body's CLU).
-template <typename T, bool MHD, int C>
-__global__ void __launch_bounds__(512, 1) fluid_seg_clu_kernel(const __grid_constant__ FluidArgs a) {
-    fluid_seg_body<T, MHD, C, VISC_NONE, true>(a, blockIdx.x);
-}
-
-template <typename T, bool MHD, int C>
-__global__ void __launch_bounds__(512, 1) fluid_seg_clu_batch_kernel(const FluidArgs* __restrict__ args,
-                                                                      const BlockMap* __restrict__ map) {
-    __shared__ FluidArgs sa;
-    const BlockMap bm = map[blockIdx.x];
-    load_member_args(sa, args + bm.member);
-    __syncthreads();
-    fluid_seg_body<T, MHD, C, VISC_NONE, true>(sa, (unsigned)bm.block);
+    fluid_seg_body<T, MHD, C, VISC_NONE, CLU, FADE>(sa, (unsigned)bm.block);
 }
 
 }  // namespace img

@@ -8,95 +8,109 @@
 
 namespace img {
 
-// Segment fluid kernels by cells per thread (2, 3, 4 and 8; FP64: 2, 3 and 4).  3 serves pencils of
-// 3 cells held whole by one thread.
-template <typename T, bool MHD>
+// Segment fluid kernels by cells per thread: 2, 3, 4 and 8 (FP64: 2, 3 and 4); 3 serves pencils of 3 cells held
+// whole by one thread.  Over a cluster (CLU) 2, 4 and 8 (FP64: 2 and 4), with fade ends 2 and 4.  FP64 CTAs
+// of at most 256 threads have kernels of their own for 3 and 4 (MAXT, fluid_seg_kernel).
+template <typename T, int MHD, bool CLU, bool FADE, int MAXT>
 void (*fluid_seg_kernel_c(int C))(const FluidArgs) {
-    if constexpr (sizeof(T) == 4) {
-        if (C == 8) return fluid_seg_kernel<T, MHD, 8>;
+    if constexpr (sizeof(T) == 4 && !FADE) {
+        if (C == 8) return fluid_seg_kernel<T, MHD, 8, VISC_NONE, CLU, FADE, MAXT>;
     }
-    if (C == 3) return fluid_seg_kernel<T, MHD, 3>;
-    return C == 2 ? fluid_seg_kernel<T, MHD, 2> : fluid_seg_kernel<T, MHD, 4>;
+    if constexpr (!CLU && !FADE) {
+        if (C == 3) return fluid_seg_kernel<T, MHD, 3, VISC_NONE, CLU, FADE, MAXT>;
+    }
+    return C == 2 ? fluid_seg_kernel<T, MHD, 2, VISC_NONE, CLU, FADE, MAXT> : fluid_seg_kernel<T, MHD, 4, VISC_NONE, CLU, FADE, MAXT>;
 }
 
-template <typename T, bool MHD>
+template <typename T, int MHD, bool CLU, bool FADE, int MAXT>
 void (*fluid_seg_batch_kernel_c(int C))(const FluidArgs*, const BlockMap*) {
-    if constexpr (sizeof(T) == 4) {
-        if (C == 8) return fluid_seg_batch_kernel<T, MHD, 8>;
+    if constexpr (sizeof(T) == 4 && !FADE) {
+        if (C == 8) return fluid_seg_batch_kernel<T, MHD, 8, CLU, FADE, MAXT>;
     }
-    if (C == 3) return fluid_seg_batch_kernel<T, MHD, 3>;
-    return C == 2 ? fluid_seg_batch_kernel<T, MHD, 2> : fluid_seg_batch_kernel<T, MHD, 4>;
+    if constexpr (!CLU && !FADE) {
+        if (C == 3) return fluid_seg_batch_kernel<T, MHD, 3, CLU, FADE, MAXT>;
+    }
+    return C == 2 ? fluid_seg_batch_kernel<T, MHD, 2, CLU, FADE, MAXT> : fluid_seg_batch_kernel<T, MHD, 4, CLU, FADE, MAXT>;
 }
 
 // With artificial viscosity: 2 and 4 cells per thread.
-template <typename T, bool MHD, int VT>
+template <typename T, int MHD, int VT, int MAXT>
 void (*fluid_seg_visc_kernel_c(int C))(const FluidArgs) {
-    return C == 2 ? fluid_seg_kernel<T, MHD, 2, VT> : fluid_seg_kernel<T, MHD, 4, VT>;
+    return C == 2 ? fluid_seg_kernel<T, MHD, 2, VT, false, false, MAXT> : fluid_seg_kernel<T, MHD, 4, VT, false, false, MAXT>;
 }
 
-template <typename T>
-void (*fluid_seg_kernel_p(int C, bool mhd, int visc = VISC_NONE))(const FluidArgs) {
-    if (visc == VISC_NR) return mhd ? fluid_seg_visc_kernel_c<T, true, VISC_NR>(C) : fluid_seg_visc_kernel_c<T, false, VISC_NR>(C);
-    if (visc == VISC_CSW) return mhd ? fluid_seg_visc_kernel_c<T, true, VISC_CSW>(C) : fluid_seg_visc_kernel_c<T, false, VISC_CSW>(C);
-    return mhd ? fluid_seg_kernel_c<T, true>(C) : fluid_seg_kernel_c<T, false>(C);
-}
-
-template <typename T>
-void (*fluid_seg_batch_kernel_p(int C, bool mhd))(const FluidArgs*, const BlockMap*) {
-    return mhd ? fluid_seg_batch_kernel_c<T, true>(C) : fluid_seg_batch_kernel_c<T, false>(C);
-}
-
-// Cluster (CLU) forms of the segment fluid kernel: 2, 4 and 8 cells per thread (FP64: 2 and 4).
-template <typename T, bool MHD>
-void (*fluid_seg_clu_kernel_c(int C))(const FluidArgs) {
-    if constexpr (sizeof(T) == 4) {
-        if (C == 8) return fluid_seg_clu_kernel<T, MHD, 8>;
+// Forms of the MHD fluxes (seg_flux): fade ends take form 2, artificial viscosity form 1, FP64 otherwise form 1 and
+// the mixed form either.
+template <typename T, int MHD, int MAXT>
+void (*fluid_seg_kernel_m(int C, bool clu, bool fade, int visc))(const FluidArgs) {
+    if constexpr (MHD < 2) {
+        if (visc == VISC_NR) return fluid_seg_visc_kernel_c<T, MHD, VISC_NR, MAXT>(C);
+        if (visc == VISC_CSW) return fluid_seg_visc_kernel_c<T, MHD, VISC_CSW, MAXT>(C);
     }
-    return C == 2 ? fluid_seg_clu_kernel<T, MHD, 2> : fluid_seg_clu_kernel<T, MHD, 4>;
+    if (fade) return fluid_seg_kernel_c<T, MHD ? 2 : 0, false, true, MAXT>(C);
+    return clu ? fluid_seg_kernel_c<T, MHD, true, false, MAXT>(C) : fluid_seg_kernel_c<T, MHD, false, false, MAXT>(C);
 }
-
-template <typename T, bool MHD>
-void (*fluid_seg_clu_batch_kernel_c(int C))(const FluidArgs*, const BlockMap*) {
+template <typename T, int MAXT>
+void (*fluid_seg_kernel_t(int C, int mhd, bool clu, bool fade, int visc))(const FluidArgs) {
     if constexpr (sizeof(T) == 4) {
-        if (C == 8) return fluid_seg_clu_batch_kernel<T, MHD, 8>;
+        if (mhd == 2 && visc == VISC_NONE) return fluid_seg_kernel_m<T, 2, MAXT>(C, clu, fade, visc);
     }
-    return C == 2 ? fluid_seg_clu_batch_kernel<T, MHD, 2> : fluid_seg_clu_batch_kernel<T, MHD, 4>;
+    return mhd ? fluid_seg_kernel_m<T, 1, MAXT>(C, clu, fade, visc) : fluid_seg_kernel_m<T, 0, MAXT>(C, clu, fade, visc);
+}
+template <typename T>
+void (*fluid_seg_kernel_p(int C, int mhd, bool clu, bool fade, int visc, unsigned block))(const FluidArgs) {
+    if constexpr (sizeof(T) == 8) {
+        if (block <= 256 && C > 2) return fluid_seg_kernel_t<T, 256>(C, mhd, clu, fade, visc);
+    }
+    return fluid_seg_kernel_t<T, 512>(C, mhd, clu, fade, visc);
+}
+
+template <typename T, int MHD, int MAXT>
+void (*fluid_seg_batch_kernel_m(int C, bool clu, bool fade))(const FluidArgs*, const BlockMap*) {
+    if (fade) return fluid_seg_batch_kernel_c<T, MHD ? 2 : 0, false, true, MAXT>(C);
+    return clu ? fluid_seg_batch_kernel_c<T, MHD, true, false, MAXT>(C) : fluid_seg_batch_kernel_c<T, MHD, false, false, MAXT>(C);
+}
+template <typename T, int MAXT>
+void (*fluid_seg_batch_kernel_t(int C, int mhd, bool clu, bool fade))(const FluidArgs*, const BlockMap*) {
+    if constexpr (sizeof(T) == 4) {
+        if (mhd == 2) return fluid_seg_batch_kernel_m<T, 2, MAXT>(C, clu, fade);
+    }
+    return mhd ? fluid_seg_batch_kernel_m<T, 1, MAXT>(C, clu, fade) : fluid_seg_batch_kernel_m<T, 0, MAXT>(C, clu, fade);
+}
+template <typename T>
+void (*fluid_seg_batch_kernel_p(int C, int mhd, bool clu, bool fade, unsigned block))(const FluidArgs*, const BlockMap*) {
+    if constexpr (sizeof(T) == 8) {
+        if (block <= 256 && C > 2) return fluid_seg_batch_kernel_t<T, 256>(C, mhd, clu, fade);
+    }
+    return fluid_seg_batch_kernel_t<T, 512>(C, mhd, clu, fade);
 }
 
 template <typename T>
-void (*fluid_seg_clu_kernel_p(int C, bool mhd))(const FluidArgs) {
-    return mhd ? fluid_seg_clu_kernel_c<T, true>(C) : fluid_seg_clu_kernel_c<T, false>(C);
-}
-
-template <typename T>
-void (*fluid_seg_clu_batch_kernel_p(int C, bool mhd))(const FluidArgs*, const BlockMap*) {
-    return mhd ? fluid_seg_clu_batch_kernel_c<T, true>(C) : fluid_seg_clu_batch_kernel_c<T, false>(C);
-}
-
-template <typename T>
-cudaError_t launch_fluid_seg(const FluidArgs& a, const PencilLaunch& L, bool mhd) {
-    if (L.clu) return launch_pencil(fluid_seg_clu_kernel_p<T>(L.seg, mhd), a, L);
-    return launch_pencil(fluid_seg_kernel_p<T>(L.seg, mhd, a.visc), a, L);
+cudaError_t launch_fluid_seg(const FluidArgs& a, const PencilLaunch& L, int mhd) {
+    return launch_pencil(fluid_seg_kernel_p<T>(L.seg, mhd, L.clu, L.fade, a.visc, L.block), a, L);
 }
 template <typename T>
-cudaError_t launch_fluid_seg_batch(const FluidArgs* args, const BlockMap* map, const PencilLaunch& L, bool mhd) {
-    if (L.clu) return launch_pencil_batch(fluid_seg_clu_batch_kernel_p<T>(L.seg, mhd), args, map, L);
-    return launch_pencil_batch(fluid_seg_batch_kernel_p<T>(L.seg, mhd), args, map, L);
+cudaError_t launch_fluid_seg_batch(const FluidArgs* args, const BlockMap* map, const PencilLaunch& L, int mhd) {
+    return launch_pencil_batch(fluid_seg_batch_kernel_p<T>(L.seg, mhd, L.clu, L.fade, L.block), args, map, L);
 }
 
 template <typename T>
 cudaError_t fluid_seg_attributes(int optin) {
     for (int C : {2, 3, 4, 8}) {
         if (sizeof(T) == 8 && C == 8) continue;
-        for (int mhd = 0; mhd < 2; ++mhd) {
-            cudaError_t e = allow_max_smem(fluid_seg_kernel_p<T>(C, mhd != 0), optin);
-            if (e == cudaSuccess) e = allow_max_smem(fluid_seg_batch_kernel_p<T>(C, mhd != 0), optin);
-            for (int vt : {VISC_NR, VISC_CSW})
-                if (e == cudaSuccess && (C == 2 || C == 4)) e = allow_max_smem(fluid_seg_kernel_p<T>(C, mhd != 0, vt), optin);
-            if (e == cudaSuccess && C != 3) e = allow_max_smem(fluid_seg_clu_kernel_p<T>(C, mhd != 0), optin);
-            if (e == cudaSuccess && C != 3) e = allow_max_smem(fluid_seg_clu_batch_kernel_p<T>(C, mhd != 0), optin);
-            if (e != cudaSuccess) return e;
-        }
+        for (int mhd = 0; mhd < 3; ++mhd)
+            for (int form = 0; form < 3; ++form) {   // plain, over a cluster, with fade ends
+                if ((form == 1 && C == 3) || (form == 2 && C != 2 && C != 4)) continue;
+                for (unsigned block : {256u, 512u}) {
+                    cudaError_t e = allow_max_smem(fluid_seg_kernel_p<T>(C, mhd, form == 1, form == 2, VISC_NONE, block), optin);
+                    if (e == cudaSuccess)
+                        e = allow_max_smem(fluid_seg_batch_kernel_p<T>(C, mhd, form == 1, form == 2, block), optin);
+                    for (int vt : {VISC_NR, VISC_CSW})
+                        if (e == cudaSuccess && form == 0 && (C == 2 || C == 4))
+                            e = allow_max_smem(fluid_seg_kernel_p<T>(C, mhd, false, false, vt, block), optin);
+                    if (e != cudaSuccess) return e;
+                }
+            }
     }
     return cudaSuccess;
 }

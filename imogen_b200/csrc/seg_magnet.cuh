@@ -19,7 +19,6 @@
 // order the exchanges through DSMEM.  A pencil of C cells is one thread's and exchanges nothing.
 #pragma once
 
-#include "lanes.cuh"
 #include "seg_fluid.cuh"
 
 namespace img {
@@ -259,32 +258,8 @@ __device__ __forceinline__ void chain_whole_lim(int lim, const V (&vr)[C], const
     else chain_whole<V, C, LIM_MINMOD>(vr, b, ff, circ_lo, circ_hi, bnew, flux);
 }
 
-// Own cells of an array: vector accesses where the segments allow (vec), else cell by cell; past the
-// pencil's end (a ragged last segment, idle threads) `fill`, and nothing stored.
-template <typename T, int C>
-__device__ __forceinline__ void win_load(const void* ptr, int o, int sd, bool vec, int nown, T fill, T (&out)[C]) {
-    const T* p = reinterpret_cast<const T*>(ptr);
-    if (vec && nown == C) {
-        seg_load<T, C>(p, o, 1, true, out);
-    } else {
-#pragma unroll
-        for (int k = 0; k < C; ++k) out[k] = k < nown ? p[o + k * sd] : fill;
-    }
-}
-template <typename T, int C>
-__device__ __forceinline__ void win_store(void* ptr, int o, int sd, bool vec, int nown, const T (&v)[C]) {
-    T* p = reinterpret_cast<T*>(ptr);
-    if (vec && nown == C) {
-        seg_store<T, C>(p, o, 1, true, v);
-    } else {
-#pragma unroll
-        for (int k = 0; k < C; ++k)
-            if (k < nown) p[o + k * sd] = v[k];
-    }
-}
-
 __device__ __forceinline__ float corner_velocity(float pm, float p, float rm, float r) { return (pm + p) * rcp_approx(rm + r); }
-__device__ __forceinline__ double corner_velocity(double pm, double p, double rm, double r) { return (pm + p) / (rm + r); }
+__device__ __forceinline__ double corner_velocity(double pm, double p, double rm, double r) { return (pm + p) * recip(rm + r); }
 
 // Chain kernel body.  Each thread reads its own C cells once (128-bit loads along x), forms their corner
 // velocities and publishes them with B_I, 16 bytes a cell and lane, cell k of every thread in plane k

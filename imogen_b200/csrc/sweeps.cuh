@@ -20,19 +20,19 @@ struct PencilLaunch {
     bool init;                 // fluid sweep / chain: captures stored edges (overrides cg)
     int seg;                   // cells per thread of the segment fluid kernel (seg_fluid.cuh) or of the window
                                // magnet kernels (seg_magnet.cuh); 0: the pencil-tile kernels
-    bool clu;                  // segment fluid kernel: one pencil along x per cluster (or per CTA with a
-                               // ragged last segment), seg_fluid.cuh's CLU form
+    bool clu;                  // segment fluid kernel: one pencil along x per cluster of CTAs, seg_fluid.cuh's
+                               // CLU form
     cudaStream_t stream;
 };
 
-template <typename T> cudaError_t launch_fluid_sweep(const FluidArgs& a, const PencilLaunch& L, bool mhd);
+template <typename T> cudaError_t launch_fluid_sweep(const FluidArgs& a, const PencilLaunch& L, int mhd);
 template <typename T> cudaError_t launch_mag_chain(const MagArgs& a, const PencilLaunch& L);
 template <typename T> cudaError_t launch_mag_ctcell(const MagArgs& a, const PencilLaunch& L);
 // The segment fluid and window magnet kernels (L.seg cells per thread), in units of their own; the
 // entry points above hand the launches with L.seg on to them.
-template <typename T> cudaError_t launch_fluid_seg(const FluidArgs& a, const PencilLaunch& L, bool mhd);
+template <typename T> cudaError_t launch_fluid_seg(const FluidArgs& a, const PencilLaunch& L, int mhd);
 template <typename T>
-cudaError_t launch_fluid_seg_batch(const FluidArgs* args, const BlockMap* map, const PencilLaunch& L, bool mhd);
+cudaError_t launch_fluid_seg_batch(const FluidArgs* args, const BlockMap* map, const PencilLaunch& L, int mhd);
 template <typename T> cudaError_t launch_mag_chain_win(const MagArgs& a, const PencilLaunch& L);
 template <typename T> cudaError_t launch_mag_ct_win(const MagArgs& a, const PencilLaunch& L);
 template <typename T> cudaError_t launch_mag_chain_win_batch(const MagArgs* args, const BlockMap* map, const PencilLaunch& L);
@@ -40,7 +40,7 @@ template <typename T> cudaError_t launch_mag_ct_win_batch(const MagArgs* args, c
 // Batched forms: one launch over the CTAs of many grids; `args` and `map` are device arrays (one
 // argument block per member, one BlockMap per CTA of the launch, L.grid_x CTAs).
 template <typename T>
-cudaError_t launch_fluid_sweep_batch(const FluidArgs* args, const BlockMap* map, const PencilLaunch& L, bool mhd);
+cudaError_t launch_fluid_sweep_batch(const FluidArgs* args, const BlockMap* map, const PencilLaunch& L, int mhd);
 // The batched fluid sweep over pencils that span a thread-block cluster (L.cluster > 1), defined in
 // fluid_cluster.cu: that translation unit is compiled at ptxas -O1 (see there), and its kernels need
 // their own shared-memory attributes (fluid_cluster_attributes).

@@ -115,7 +115,7 @@ void (*chain_batch_kernel(int cpt, int nqc, int v))(const MagArgs*, const BlockM
 inline int ct_variant(bool fade, bool cg) { return (fade ? 1 : 0) | (cg ? 2 : 0); }
 
 template <typename T>
-cudaError_t launch_fluid_sweep_batch(const FluidArgs* args, const BlockMap* map, const PencilLaunch& L, bool mhd) {
+cudaError_t launch_fluid_sweep_batch(const FluidArgs* args, const BlockMap* map, const PencilLaunch& L, int mhd) {
     if (L.seg) return launch_fluid_seg_batch<T>(args, map, L, mhd);
     if (L.cluster > 1) return launch_fluid_sweep_batch_cluster<T>(args, map, L, mhd);
     return launch_pencil_batch(fluid_batch_kernel<T>(L.cpt, mhd, kernel_variant(L.fade, L.cg, L.init)), args, map, L);
@@ -172,7 +172,7 @@ cudaError_t launch_mag_ctcell_batch(const MagArgs* args, const BlockMap* map, co
 }
 
 template <typename T>
-cudaError_t launch_fluid_sweep(const FluidArgs& a, const PencilLaunch& L, bool mhd) {
+cudaError_t launch_fluid_sweep(const FluidArgs& a, const PencilLaunch& L, int mhd) {
     if (L.seg) return launch_fluid_seg<T>(a, L, mhd);
     return launch_pencil(fluid_kernel<T>(L.cpt, mhd, kernel_variant(L.fade, L.cg, L.init)), a, L);
 }

@@ -324,8 +324,8 @@ int img_autotune(img_ctx* ctx, int trials);
  * (after img_autotune the magnet CT pass may run on a tiling of its own);
  * out = {pencils per CTA, threads per pencil, CTAs per cluster, threads per CTA, cells per thread,
  * transverse components per CTA (magnet: 1 or 2; fluid: 1), segment layout: 1 when each thread owns
- * consecutive cells -- the segment fluid kernel or the window magnet kernels, used for the steady sweeps
- * of single-CTA pencils whose shifts are circ or const -- and 0 for the pencil-tile kernels}. */
+ * consecutive cells -- the segment fluid kernel (sweeps whose ends are circ, const or fade, after a run's
+ * first) or the window magnet kernels (circ or const) -- and 0 for the pencil-tile kernels}. */
 int img_get_tiling(const img_ctx* ctx, int dim, int out[7]);
 /* Set the tiling of slot dim to one of those the autotuner may pick (same field order); a magnet
  * slot sets the chain's and the CT pass's tiling. */
