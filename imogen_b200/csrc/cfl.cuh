@@ -239,7 +239,11 @@ __device__ __forceinline__ void cfl_finalize_body(DevTime* tm, int check_running
     if (tm->dt_hist && k >= 0 && k < tm->dt_hist_cap) tm->dt_hist[k] = dt;
 }
 
+// One thread's work between two sweeps: the next kernel may be placed on the chip right away (it waits for this
+// one before it reads anything), and this one's own launch overlaps the sweep before it.
 __global__ void cfl_finalize_kernel(DevTime* tm, int check_running) {
+    pdl_trigger();
+    pdl_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     cfl_finalize_body(tm, check_running);
 }

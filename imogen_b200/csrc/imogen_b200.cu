@@ -1209,8 +1209,14 @@ int time_update_async(img_ctx* ctx, int flux_direction) {
         ctx->cfl_valid = false;
         return IMG_OK;
     }
-    cfl_finalize_kernel<<<1, 32, 0, ctx->stream>>>(ctx->tm, flux_direction == 1 ? 1 : 0);
-    CK(cudaGetLastError());
+    PencilLaunch L{};
+    L.grid_x = L.grid_y = 1;
+    L.block = 32;
+    L.cluster = 1;
+    L.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t lc = pencil_config(L, attr);   // programmatic stream serialization, as the pencil kernels
+    CK(cudaLaunchKernelEx(&lc, cfl_finalize_kernel, ctx->tm, flux_direction == 1 ? 1 : 0));
     ctx->launches += 1;
     ctx->cfl_valid = false;
     return IMG_OK;
