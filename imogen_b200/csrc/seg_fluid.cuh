@@ -166,15 +166,18 @@ __device__ __forceinline__ void win_store(void* ptr, int o, int sd, bool vec, in
 struct SegPressure {
     double g, g1, half_g1, p_ms;
     __device__ __forceinline__ explicit SegPressure(double G) : g(G), g1(G - 1.0), half_g1((G - 1.0) * 0.5), p_ms(0.5 * (2.0 - G)) {}
-    // P and rho c_s^2 from p0 = (G-1)(E - rho v^2/2) and msq = B^2
+    // P and rho c_s^2 from x = E - rho v^2/2 and msq = B^2.  Each B^2 term is rounded before it joins (G-1) x, as
+    // the pencil-tile kernels' pressure_totsnd_mixed comes out, whose FP64 bits the mixed form shares: one of the
+    // other orders differs in the last FP64 bit of every other cell, hence in the FP32 pressure of one in 2e9, and a
+    // 256^3 shear run grows that to 1e-3 of B's scale at single cells in 120 iterations.
     template <int MSQ>
-    __device__ __forceinline__ void totals(double p0, double msq, double& pt, double& c2) const {
+    __device__ __forceinline__ void totals(double x, double msq, double& pt, double& c2) const {
         if constexpr (MSQ) {
-            c2 = fma(2.0, msq, g * fma(-half_g1, msq, p0));
-            pt = fma(p_ms, msq, p0);
+            c2 = fma(g, fma(g1, x, -(half_g1 * msq)), 2.0 * msq);
+            pt = fma(g1, x, p_ms * msq);
         } else {
-            c2 = g * p0;
-            pt = p0;
+            pt = g1 * x;
+            c2 = g * pt;
         }
     }
 };
@@ -192,7 +195,7 @@ __device__ __forceinline__ float seg_pressure(const SegPressure& k, const float 
     const double px = u[1], py = u[2], pz = u[3];
     const double psq = fma(pz, pz, fma(px, px, py * py));
     double c2, pt;
-    k.totals<MSQ>(k.g1 * fma(-(0.5 * psq), inv, (double)u[4]), msq, pt, c2);
+    k.totals<MSQ>(fma(-(0.5 * psq), inv, (double)u[4]), msq, pt, c2);
     cs = sqrt_approx(fabsf((float)(c2 * inv)));
     p = pt < 0 ? 0.f : (float)pt;
     return fabsf(u[1] * ir) + cs;
@@ -203,7 +206,7 @@ __device__ __forceinline__ double seg_pressure(const SegPressure& k, const doubl
     ir = recip(u[0]);
     const double psq = fma(u[3], u[3], fma(u[1], u[1], u[2] * u[2]));
     double c2, pt;
-    k.totals<MSQ>(k.g1 * fma(-(0.5 * psq), ir, u[4]), msq, pt, c2);
+    k.totals<MSQ>(fma(-(0.5 * psq), ir, u[4]), msq, pt, c2);
     cs = sqrt_goldschmidt(fabs(c2 * ir));
     p = pt < 0 ? 0.0 : pt;
     return fabs(u[1] * ir) + cs;

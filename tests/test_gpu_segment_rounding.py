@@ -1,0 +1,56 @@
+"""The FP32 rounding of the segment fluid kernels (GPU required).  The flows these grids carry grow a difference in the
+last bit by several powers of ten in a hundred iterations, so a kernel that replaces another on the same grid has to
+round as it did: one sweep of the segment kernels equals one of the pencil-tile kernels (IMOGEN_B200_TILE_KERNELS=1)
+bit for bit."""
+import numpy as np
+import pytest
+
+from imogen_b200 import ImogenRun
+
+pytestmark = pytest.mark.gpu
+F32 = lambda a: np.asarray(a, dtype=np.float32).astype(np.float64)
+
+
+def _settings(grid, bc, magnet):
+    return dict(grid=grid, dgrid=(1 / 256,) * 3, gamma=5 / 3, cfl=0.35, bc=bc, limiter="vanleer", magnet=magnet,
+                time_max=1e5, iter_max=10 ** 6)
+
+
+def _sweep(settings, state, X, dt, tile, monkeypatch):
+    """One fluid sweep along X, not a run's first (the first capture takes the tile kernels on either side)."""
+    monkeypatch.setenv("IMOGEN_B200_TILE_KERNELS", "1" if tile else "0")
+    r = ImogenRun(precision="mixed", **settings)
+    assert bool(r.tiling("fluid")[X][6]) != tile
+    r.set_state(*state(r))
+    r.time.set(0.0, 0.0, 1)
+    r.relaxing_fluid(2 if X == 1 else 1)   # with dt = 0: changes nothing
+    r.time.set(0.0, dt, 1)
+    r.relaxing_fluid(X)
+    out = [r.download(k).astype(np.float32) for k in ("mass", "momx", "momy", "momz", "ener")]
+    r.close()
+    return out
+
+
+def _pressure_residue(grid, X, seed):
+    """A state at rest along X whose 'totsnd' pressure is what the FP32 rounding of E leaves of terms 1e7 times
+    larger.  With a tiny dt the new momentum along X shows the FP32 pressure alone, and an FP64 sum rounded in another
+    order shows in a few cells of a hundred."""
+    def state(run):
+        rng = np.random.default_rng(seed)
+        rho, mom, mag = F32(rng.uniform(0.5, 2, grid)), F32(rng.uniform(-1, 1, (3,) + grid)), F32(rng.uniform(-1, 1, (3,) + grid))
+        mom[X - 1] = mag[X - 1] = 0
+        run.set_state(rho, mom, rho, mag)   # for the cell-centred field
+        msq = sum(run.download(k) ** 2 for k in ("cmagx", "cmagy", "cmagz"))
+        at = 0.5 * (mom ** 2).sum(0) / rho - msq / 4   # (gamma - 1) (E - kinetic) + (2 - gamma) B^2 / 2 = 0
+        ener = F32(at)
+        return rho, mom, np.where(ener < at, F32(np.nextafter(ener.astype(np.float32), np.float32(9))), ener), mag
+    return state
+
+
+@pytest.mark.parametrize("bc", ["circ", "const"])
+@pytest.mark.parametrize("grid,X", [((64, 64, 16), 1), ((64, 64, 16), 2), ((16, 16, 64), 3), ((75, 32, 9), 1), ((32, 75, 9), 2)])
+def test_pressure_rounds_as_in_the_tile_kernels(grid, X, bc, monkeypatch):
+    s = _settings(grid, bc, True)
+    a, b = (_sweep(s, _pressure_residue(grid, X, 7), X, 1e-20, tile, monkeypatch) for tile in (False, True))
+    assert np.count_nonzero(a[X]) > 0.9 * a[X].size
+    assert all((x == y).all() for x, y in zip(a, b)), [int((x != y).sum()) for x, y in zip(a, b)]
