@@ -688,13 +688,14 @@ __device__ __forceinline__ void seg_correct_all(const SegEnds& e, const T (&u)[5
 
 // ---- fade ends (fade_shift.m:21-45) ---------------------------------------------------------------------
 // The damping of one cell's row in a shifted array: v toward the shifted array's first value (s0, weight
-// lo), then toward its last (sN, weight hi); weights are 0 (and nothing is done) away from the ends.
+// lo), then toward its last (sN, weight hi); weights are 0 (and nothing is done) away from the ends.  The share of v
+// is rounded first, and in FP32 the half step's change too except the energy's, as in the pencil-tile kernels.
 template <typename T>
 struct SegFade {
     T lo, hi;
     __device__ __forceinline__ T operator()(T v, T s0, T sN) const {
-        if (lo != T(0)) v = v_fma(T(1) - lo, v, lo * s0);
-        if (hi != T(0)) v = v_fma(T(1) - hi, v, hi * sN);
+        if (lo != T(0)) v = v_fma(lo, s0, (T(1) - lo) * v);
+        if (hi != T(0)) v = v_fma(hi, sN, (T(1) - hi) * v);
         return v;
     }
 };
@@ -976,7 +977,8 @@ __device__ __forceinline__ void fluid_seg_body(const FluidArgs& a, unsigned vblo
 #pragma unroll
             for (int k = 0; k < C; ++k) {
                 const T Rm = fade_lo ? fw[k](R[k], R0, RN) : R[k], Lp = fade_hi ? fw[k](L[k + 1], L0, LN) : L[k + 1];
-                u[v][k] = v_fma(-hfc, R[k + 1] - Rm + L[k] - Lp, u[v][k]);
+                const T change = R[k + 1] - Rm + L[k] - Lp;
+                u[v][k] = sizeof(T) == 4 && v < 4 ? u[v][k] - hfc * change : v_fma(-hfc, change, u[v][k]);
             }
         }
     }

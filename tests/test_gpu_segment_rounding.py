@@ -54,3 +54,22 @@ def test_pressure_rounds_as_in_the_tile_kernels(grid, X, bc, monkeypatch):
     a, b = (_sweep(s, _pressure_residue(grid, X, 7), X, 1e-20, tile, monkeypatch) for tile in (False, True))
     assert np.count_nonzero(a[X]) > 0.9 * a[X].size
     assert all((x == y).all() for x, y in zip(a, b)), [int((x != y).sum()) for x, y in zip(a, b)]
+
+
+def _ordinary(grid, magnet, seed):
+    def state(run):
+        rng = np.random.default_rng(seed)
+        rho, mom = rng.uniform(0.5, 2, grid), rng.uniform(-1, 1, (3,) + grid)
+        mag = rng.uniform(-1, 1, (3,) + grid) if magnet else np.zeros((3,) + grid)
+        return rho, mom, 1 + 0.5 * (mom ** 2).sum(0) / rho + 0.5 * (mag ** 2).sum(0), mag
+    return state
+
+
+@pytest.mark.parametrize("magnet", [False, True])
+@pytest.mark.parametrize("grid,bc,X", [((48, 40, 1), "fade", 1), ((48, 41, 1), "fade", 2), ((24, 22, 67), "fade", 3), ((500, 24, 1), "fade", 1),
+                                       ((61, 40, 1), {"x": ("fade", "const"), "y": "fade", "z": "circ"}, 1),
+                                       ((40, 61, 1), {"x": "fade", "y": ("circ", "fade"), "z": "circ"}, 2)])
+def test_fade_ends_round_as_in_the_tile_kernels(grid, bc, X, magnet, monkeypatch):
+    s = _settings(grid, bc, magnet)
+    a, b = (_sweep(s, _ordinary(grid, magnet, 5), X, 1e-3, tile, monkeypatch) for tile in (False, True))
+    assert all((x == y).all() for x, y in zip(a, b)), [int((x != y).sum()) for x, y in zip(a, b)]
