@@ -130,30 +130,50 @@ template <typename T> __device__ __forceinline__ T tmax(T a, T b) { return a > b
 __device__ __forceinline__ double msign(double v) { return v > 0 ? 1.0 : (v < 0 ? -1.0 : (v == 0 ? 0.0 : v)); }
 __device__ __forceinline__ float msign(float v) { return v > 0 ? 1.f : (v < 0 ? -1.f : (v == 0 ? 0.f : v)); }
 
-// FP64 reciprocal of a normal x by one third-order Newton-Raphson (Householder) step, r (1 + e + e^2) with
-// e = 1 - x r, from the hardware's estimate (PTX rcp.approx.ftz.f64, relative error below 2^-19, so the step
-// leaves less than 2^-57 before rounding): within 1 ulp, 4 instructions and no branch, where the correctly
-// rounded division takes about 30 and a branch for the special cases.  Each FP64 cell of a fluid sweep divides
-// some 14 times, which made its integer and control instructions outnumber the FP64 ones three to one.
+// FP64 reciprocal, quotient and square root from the hardware's estimates (PTX rcp.approx.ftz.f64 and
+// rsqrt.approx.ftz.f64, relative errors below 2^-19) with multiplications and FMAs only: the compiler's division
+// takes about 30 instructions and a branch for the special cases, and each FP64 cell of a fluid sweep divides some
+// 14 times, so integer and control instructions outnumbered the FP64 ones three to one.  Each ends in a residual
+// step (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990): from an
+// approximation within 1 ulp, the residual of one FMA is exact and the corrected result correctly rounded (a
+// mantissa of ones excepted, whose reciprocal lies too close to half-way).
+
+// 1/x of a normal x within 1 ulp: one third-order Newton-Raphson (Householder) step r (1 + e + e^2), e = 1 - x r.
 __device__ __forceinline__ double rcp_newton(double x) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
     const double e = fma(-x, r, 1.0);
     return fma(r, fma(e, e, e), r);
 }
-// Whether |x| lies in [2^-1000, 2^1000): the estimates below neither flush nor overflow there.
+// Whether |x| lies in [2^-1000, 2^1000), where the estimates neither flush nor overflow, and its low word is not all
+// ones, as that of a mantissa of ones is.
 __device__ __forceinline__ bool mid_range(double x) {
     const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
-    return h - 0x01700000u < 0x7d000000u;
+    return h - 0x01700000u < 0x7d000000u && __double2loint(x) != -1;
 }
-// 1/x for any x: the step above, or the division where |x| is extreme, zero, infinite or NaN.
+// 1/x for any x: the division where |x| is extreme, zero, infinite, NaN or has a mantissa of ones.
 __device__ __forceinline__ double recip(double x) {
-    if (mid_range(x)) return rcp_newton(x);
-    return 1.0 / x;
+    if (!mid_range(x)) return 1.0 / x;
+    const double r = rcp_newton(x);
+    return fma(r, fma(-x, r, 1.0), r);
 }
-// Square root of x >= 0: Goldschmidt's iteration with a final residual correction (Markstein, "Software
-// division and square root using Goldschmidt's algorithms", 2004) from the hardware's reciprocal square root
-// estimate; the library's function for extreme, zero, infinite and NaN x.  Within 1 ulp.
+// a/b from r, 1/b correctly rounded (or within 1 ulp: then a/b within 2^-50 ulp of half-way may round to the farther
+// side); an infinite estimate (a infinite, or an overflow) stays as it is.
+__device__ __forceinline__ double quotient_from(double a, double b, double r) {
+    const double q = a * r;
+    return fabs(q) < __longlong_as_double(0x7ff0000000000000ll) ? fma(fma(-q, b, a), r, q) : q;
+}
+// a/b for any a and b.
+__device__ __forceinline__ double quotient(double a, double b) {
+    return mid_range(b) ? quotient_from(a, b, recip(b)) : a / b;
+}
+// a/b from the correctly rounded inv = 1/b (dt over a grid spacing).
+__device__ __forceinline__ double quotient_by(double a, double b, double inv) {
+    const double q = a * inv;
+    return fma(fma(-q, b, a), inv, q);
+}
+// Square root of x >= 0: Goldschmidt's iteration (Markstein, "Software division and square root using Goldschmidt's
+// algorithms", 2004), two residual steps; the library's function for extreme, zero, infinite and NaN x.
 __device__ __forceinline__ double sqrt_goldschmidt(double x) {
     if (!mid_range(x)) return sqrt(x);
     double y;
@@ -162,6 +182,8 @@ __device__ __forceinline__ double sqrt_goldschmidt(double x) {
     double r = fma(-g, h, 0.5);
     g = fma(g, r, g);
     h = fma(h, r, h);
+    h = fma(h, fma(-g, h, 0.5), h);
+    g = fma(fma(-g, g, x), h, g);
     return fma(fma(-g, g, x), h, g);
 }
 
@@ -178,8 +200,9 @@ __device__ __forceinline__ T limiter_corr_t(T dL, T dR) {
             st = __fdividef(num, dL + dR);   // mixed form: fast divide
             return isnan(st) ? T(0) : st;
         } else {
-            // a positive product keeps |dL + dR| above 2^-538: the reciprocal's operand is normal
-            st = num * rcp_newton(dL + dR);
+            // a positive product keeps |dL + dR| above 2^-538: the reciprocal's operand is normal (and, beyond 2^1022,
+            // flushed: the correction is 0)
+            st = quotient_from(num, dL + dR, rcp_newton(dL + dR));
             return num > T(0) && !isnan(st) ? st : T(0);
         }
     } else {
@@ -329,11 +352,10 @@ __device__ __forceinline__ PressOutF pressure_totsnd_mixed(double G, float rho, 
 // 'sound' speed of pressure.m): one FP64 reciprocal of rho serves the four quotients.
 __device__ __forceinline__ void cfl_speeds(double G, double rho, double px, double py, double pz, double E,
                                            double msq, double s[3]) {
-    const double inv = recip(rho);
-    const double vsq = (px * px + py * py + pz * pz) * (inv * inv);
-    double r = (G - 1.0) * (E - 0.5 * rho * vsq);
-    r = r - (G - 1.0) * 0.5 * msq;
-    const double cs = sqrt_goldschmidt(fabs((G * r + 2.0 * msq) * inv));
+    const double inv = recip(rho), g1 = G - 1.0;   // (FMAs written out: the units differ in contracting sums)
+    const double vsq = fma(pz, pz, fma(px, px, py * py)) * (inv * inv);
+    const double r = fma(g1, fma(-(0.5 * rho), vsq, E), -(g1 * 0.5 * msq));
+    const double cs = sqrt_goldschmidt(fabs(fma(G, r, 2.0 * msq) * inv));
     s[0] = fabs(px * inv) + cs;
     s[1] = fabs(py * inv) + cs;
     s[2] = fabs(pz * inv) + cs;

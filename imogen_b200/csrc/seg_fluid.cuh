@@ -811,7 +811,7 @@ __device__ __forceinline__ void fluid_seg_body(const FluidArgs& a, unsigned vblo
     constexpr bool LOADB = MHD || VT == VISC_CSW;   // cswSoundSpeed reads every cell-centred component
     pdl_wait();
     const int stop = a.tm->done | (!CLU || g.CL == 1 ? a.tm->error : 0);   // cluster launches return on `done` only
-    const double dt = a.tm->dt, dq = dt * a.inv_dx, dtx = fma(fma(-dq, a.dx, dt), a.inv_dx, dq);   // dt / dx, one residual step
+    const double dtx = quotient_by(a.tm->dt, a.dx, a.inv_dx);
     T u[5][C], bb[3][C], F[5][C];
     auto load_u = [&](int v, T (&w)[C]) { win_load<T, C, true>(qv[v], o0, sd, vec, nown, v == 0 ? T(1) : T(0), w); };
     auto load_b = [&]() {   // the cell-centred B, which a fluid sweep leaves alone

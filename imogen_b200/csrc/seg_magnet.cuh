@@ -259,7 +259,7 @@ __device__ __forceinline__ void chain_whole_lim(int lim, const V (&vr)[C], const
 }
 
 __device__ __forceinline__ float corner_velocity(float pm, float p, float rm, float r) { return (pm + p) * rcp_approx(rm + r); }
-__device__ __forceinline__ double corner_velocity(double pm, double p, double rm, double r) { return (pm + p) * recip(rm + r); }
+__device__ __forceinline__ double corner_velocity(double pm, double p, double rm, double r) { return quotient(pm + p, rm + r); }
 
 // Chain kernel body.  Each thread reads its own C cells once (128-bit loads along x), forms their corner
 // velocities and publishes them with B_I, 16 bytes a cell and lane, cell k of every thread in plane k
@@ -295,7 +295,7 @@ __device__ __forceinline__ void mag_chain_win_body(const MagArgs& a, unsigned vb
     pdl_wait();
     const DevTime* tm = a.tm;
     const int stop = tm->done | (g.CL == 1 ? tm->error : 0);   // clusters: as in the fluid sweeps
-    const T ff = (T)(0.5 * tm->dt * a.inv_dx);
+    const T ff = (T)quotient_by(0.5 * tm->dt, a.dx, a.inv_dx);
 
     // ---- own cells: the corner velocity (magnetFlux.m:18-19) and B_I of both components ------------
     T vgo[2][C], bo[2][C];
@@ -496,7 +496,7 @@ __device__ __forceinline__ void mag_ct_win_body(const MagArgs& a, unsigned vbloc
     }
     win_barrier(g);   // every thread has read B_X before any writes it
     // D_q = C_q.shift(X,-1); B_X = (B_X - dt/dI1 D_1) - dt/dI2 D_2 at the own cells and the one after them
-    const T f0 = (T)(dt * a.inv_dI[0]), f1 = (T)(dt * a.inv_dI[1]);
+    const T f0 = (T)quotient_by(dt, a.dI[0], a.inv_dI[0]), f1 = (T)quotient_by(dt, a.dI[1], a.inv_dI[1]);
     T bx[C], cbx[C], cb2[C];
 #pragma unroll
     for (int k = 0; k < C; ++k) bx[k] = v_fma(-f1, Cq[1][k], v_fma(-f0, Cq[0][k], bxo[k]));
