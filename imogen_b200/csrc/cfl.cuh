@@ -202,7 +202,10 @@ __global__ void rad_init_finalize_kernel(DevTime* tm, double scale) {
 // check_running: evaluate TimeManager.running (time < TIMEMAX) first, as imogen.m:58 does at the
 // top of each iteration; the iteration limit is enforced by the host.
 __device__ __forceinline__ void cfl_finalize_body(DevTime* tm, int check_running) {
-    if (tm->done || tm->error) return;
+    if (tm->done || tm->error) {
+        if (tm->error) tm->halt = 1;
+        return;
+    }
     if (check_running && !(tm->time < tm->time_max)) {
         tm->done = 1;
         return;
@@ -219,6 +222,7 @@ __device__ __forceinline__ void cfl_finalize_body(DevTime* tm, int check_running
     tm->grid_index = gi;
     if (gi < 1) {   // TimeManager.m:79-86 (fireCFLError)
         tm->error |= DERR_CFL;
+        tm->halt = 1;
         return;
     }
     double dt = tm->cfl * tm->dgrid[gi - 1] / cmax;
@@ -229,6 +233,7 @@ __device__ __forceinline__ void cfl_finalize_body(DevTime* tm, int check_running
     }
     if (!isfinite(dt)) {
         tm->error |= DERR_NONFINITE_DT;
+        tm->halt = 1;
         return;
     }
     tm->dt = dt;

@@ -72,7 +72,7 @@ struct DevTime {
     int error;              // DevError bits
     int done;               // TimeManager.running turned false (time >= TIMEMAX)
     int iters_run;          // iterations that started (TimeManager.running was true at their top)
-    int reserved1;
+    int halt;               // a time update found an error: set between sweeps, so every CTA of a cluster sees the same
     unsigned long long maxbits[3];   // per-direction max of |v_i| + c_s (bit pattern, >= 0)
     unsigned int counter;            // CTAs finished in the current CFL reduction
     unsigned int pad2;

@@ -2092,6 +2092,7 @@ int img_set_time(img_ctx* ctx, double time, double dt, int iteration) {
     ctx->host_tm->dt = dt;
     ctx->host_tm->done = 0;
     ctx->host_tm->error = 0;
+    ctx->host_tm->halt = 0;
     ctx->host_tm->iters_run = iteration - 1;
     CK(cudaMemcpyAsync(ctx->tm, ctx->host_tm, sizeof(DevTime), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));

@@ -810,7 +810,7 @@ __device__ __forceinline__ void fluid_seg_body(const FluidArgs& a, unsigned vblo
     const int nx = d == 0 ? 0 : (d1 == 0 ? 1 : 2), ny = d == 1 ? 0 : (d1 == 1 ? 1 : 2), nz = d == 2 ? 0 : (d1 == 2 ? 1 : 2);
     constexpr bool LOADB = MHD || VT == VISC_CSW;   // cswSoundSpeed reads every cell-centred component
     pdl_wait();
-    const int stop = a.tm->done | (!CLU || g.CL == 1 ? a.tm->error : 0);   // cluster launches return on `done` only
+    const int stop = a.tm->done | (!CLU || g.CL == 1 ? a.tm->error : a.tm->halt);   // (clusters: fluid_sweep_body_general)
     const double dtx = quotient_by(a.tm->dt, a.dx, a.inv_dx);
     T u[5][C], bb[3][C], F[5][C];
     auto load_u = [&](int v, T (&w)[C]) { win_load<T, C, true>(qv[v], o0, sd, vec, nown, v == 0 ? T(1) : T(0), w); };

@@ -294,7 +294,7 @@ __device__ __forceinline__ void mag_chain_win_body(const MagArgs& a, unsigned vb
     const int o0 = wp.base + r0 * sd;
     pdl_wait();
     const DevTime* tm = a.tm;
-    const int stop = tm->done | (g.CL == 1 ? tm->error : 0);   // clusters: as in the fluid sweeps
+    const int stop = tm->done | (g.CL == 1 ? tm->error : tm->halt);   // clusters: as in the fluid sweeps
     const T ff = (T)quotient_by(0.5 * tm->dt, a.dx, a.inv_dx);
 
     // ---- own cells: the corner velocity (magnetFlux.m:18-19) and B_I of both components ------------
@@ -464,7 +464,7 @@ __device__ __forceinline__ void mag_ct_win_body(const MagArgs& a, unsigned vbloc
     const bool end_hi = !circ_hi && past;
     pdl_wait();
     const DevTime* tm = a.tm;
-    const int stop = tm->done | (g.CL == 1 ? tm->error : 0);   // clusters: as in the fluid sweeps
+    const int stop = tm->done | (g.CL == 1 ? tm->error : tm->halt);   // clusters: as in the fluid sweeps
     const double dt = tm->dt;
     T* BX = reinterpret_cast<T*>(a.w_BX);
     // C_q = F_q - F_q.shift(I_q, +1) (relaxingMagnet.m:56) at cells -1 .. C-1 (index j + 1)
