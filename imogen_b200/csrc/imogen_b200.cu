@@ -446,7 +446,7 @@ std::vector<PencilCfg> seg_candidates(const Geom& g, int d, size_t elem, bool vi
     const int N = g.n[d];
     const long long ncol = g.ncell / N;
     auto add = [&](int Wb, int S, int CL, int NT, int C) {
-        if (seg_smem(elem, NT, Wb, visc, !visc && CL == 1) > kPencilSmemLimit) return;
+        if (seg_smem(elem, NT, Wb, visc, false) > kPencilSmemLimit) return;
         PencilCfg p;
         p.Wb = Wb;
         p.G = S;
@@ -488,7 +488,7 @@ std::vector<PencilCfg> seg_candidates(const Geom& g, int d, size_t elem, bool vi
 // cells per thread, S = ceil(N / C) threads per pencil (the last segment may be shorter), whole pencils in one
 // CTA of NT = Wb * S threads rounded up to a multiple of 32 (32 <= NT <= 512, the threads past the segments
 // idle); along y and z Wb >= 4 pencils side by side (2 where 4 do not fit; up to 64, or to the CTA where each
-// pencil is one thread's).  Along x, for S above 256 (512) segments, one pencil over a cluster of
+// pencil is one thread's), along x up to 64, or to the CTA where the last segment is shorter.  Along x, for S above 256 (512) segments, one pencil over a cluster of
 // CL = ceil(S / 256) <= 8 CTAs (ceil(S / 512) <= 4) of NT = ceil(S / CL) rounded up.
 std::vector<PencilCfg> win_candidates(const Geom& g, int d) {
     std::vector<PencilCfg> out;
@@ -507,7 +507,8 @@ std::vector<PencilCfg> win_candidates(const Geom& g, int d) {
     for (int C : {2, 3, 4, 8}) {
         if (C == 3 && N % 3 != 0) continue;
         const int S = (N + C - 1) / C;
-        for (int Wb = d == 0 ? 1 : (4 * S <= 512 ? 4 : 2); Wb <= (d != 0 && S == 1 ? 512 : 64); Wb *= 2) {
+        const int most = (d == 0 ? N % C != 0 : S == 1) ? 512 : 64;
+        for (int Wb = d == 0 ? 1 : (4 * S <= 512 ? 4 : 2); Wb <= most; Wb *= 2) {
             const int NT = std::max(32, (Wb * S + 31) / 32 * 32);
             if (NT > 512) break;
             if (Wb > 1 && (long long)Wb / 2 >= ncol && Wb * S > 32) break;
@@ -575,7 +576,9 @@ PencilCfg choose_window(const Geom& g, int d, size_t elem, const PencilCfg& tile
 // exchange records fit an SM (192 threads; 96^3 x 50 us, y 57 us), else 4 (96^3: 62 and 65 us; 128^3 y: 137 us,
 // with 2 cells in 256 threads 199 us).
 PencilCfg choose_fluid(const Geom& g, int d, size_t elem, const PencilCfg& tile) {
-    std::vector<PencilCfg> c = seg_candidates(g, d, elem);
+    std::vector<PencilCfg> c = seg_candidates(g, d, elem);   // with room for the anchors of fade ends
+    c.erase(std::remove_if(c.begin(), c.end(),
+                           [&](const PencilCfg& p) { return seg_smem(elem, p.NT, p.Wb, false, p.CL == 1) > kPencilSmemLimit; }), c.end());
     // (longer pencils keep 4: their CTAs have the warps, and tubes of an ensemble fill the chip together)
     const PencilCfg* best = small_grid(g) && g.n[d] <= 256 ? default_segments(c, g, d, elem, 2, 128, 2.0) : nullptr;
     if (!best && elem == 8) {
@@ -772,12 +775,13 @@ int launch_fluid(img_ctx* ctx, int d, bool cfl) {
     FluidArgs a{};
     const img_config& c = ctx->cfg;
     // the segment kernel takes the sweeps whose ends are circ, const or fade, the same for all fluid classes
-    // (fade: pencils of one CTA, 2 or 4 cells per thread); stored-edge capture (a run's first sweep) and
-    // other ends take the tile kernels
+    // (fade: pencils of one CTA, 2 or 4 cells per thread, with room for the anchors); stored-edge capture (a
+    // run's first sweep) and other ends take the tile kernels
     const bool fade = fade_on(c, d, CLS_MASS, CLS_ENER);
     const bool init = ctx->init_store || ctx->init_flux;
     const PencilCfg& ps = ctx->pcfg[0][d];
-    bool seg_ok = ps.seg && !init && !(fade && (ps.CL > 1 || (ps.seg != 2 && ps.seg != 4)));
+    bool seg_ok = ps.seg && !init &&
+                  !(fade && (ps.CL > 1 || (ps.seg != 2 && ps.seg != 4) || seg_smem(sizeof(T), ps.NT, ps.Wb, false, true) > kPencilSmemLimit));
     for (int k = 0; k < 3; ++k)
         for (int side = 0; side < 2; ++side)
             if (!copy_ghost_mode(c.bc_modes[k][side][d]) || c.bc_modes[k][side][d] != c.bc_modes[CLS_MASS][side][d]) seg_ok = false;
