@@ -157,11 +157,15 @@ __device__ __forceinline__ double recip(double x) {
     const double r = rcp_newton(x);
     return fma(r, fma(-x, r, 1.0), r);
 }
-// a/b for any a and b; an infinite estimate (a infinite, or an overflow) stays as it is.
-__device__ __forceinline__ double quotient(double a, double b) {
-    if (!mid_range(b)) return a / b;
-    const double r = recip(b), q = a * r;
+// a/b from r, 1/b correctly rounded (or within 1 ulp: then a/b within 2^-50 ulp of half-way may round to the farther
+// side); an infinite estimate (a infinite, or an overflow) stays as it is.
+__device__ __forceinline__ double quotient_from(double a, double b, double r) {
+    const double q = a * r;
     return fabs(q) < __longlong_as_double(0x7ff0000000000000ll) ? fma(fma(-q, b, a), r, q) : q;
+}
+// a/b for any a and b.
+__device__ __forceinline__ double quotient(double a, double b) {
+    return mid_range(b) ? quotient_from(a, b, recip(b)) : a / b;
 }
 // a/b from the correctly rounded inv = 1/b (dt over a grid spacing).
 __device__ __forceinline__ double quotient_by(double a, double b, double inv) {
@@ -190,24 +194,16 @@ template <int LIM, typename T>
 __device__ __forceinline__ T limiter_corr_t(T dL, T dR) {
     if constexpr (LIM == LIM_VANLEER) {
         T p = dL * dR;
+        T num = p > T(0) ? p : T(0);
+        T st;
         if constexpr (sizeof(T) == 4) {
-            T num = p > T(0) ? p : T(0);
-            T st = __fdividef(num, dL + dR);   // mixed form: fast divide
+            st = __fdividef(num, dL + dR);   // mixed form: fast divide
             return isnan(st) ? T(0) : st;
         } else {
-            // p / (dL + dR) where p > 0, within 0.5 ulp and 2^-21 ulp: the estimate, one Newton step, the quotient
-            // and its residual; the sign and the range of p
-            // are read off its high word, without FP64 comparisons.  A positive p keeps |dL + dR| above 2^-538: the operand is
-            // normal (and, beyond 2^1022, flushed: 0).
-            const double s = dL + dR;
-            double r;
-            asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(s));
-            r = fma(r, fma(-s, r, 1.0), r);
-            double st = p * r;
-            st = fma(fma(-st, s, p), r, st);
-            const int h = __double2hiint(p);
-            if (h >= 0x7ff00000) st = p == p && !isinf(s) ? copysign(p, s) : 0.0;   // the product overflows
-            return h > 0 ? st : 0.0;   // (a positive p below 2^-1042 counts as 0)
+            // a positive product keeps |dL + dR| above 2^-538: the reciprocal's operand is normal (and, beyond 2^1022,
+            // flushed: the correction is 0)
+            st = quotient_from(num, dL + dR, rcp_newton(dL + dR));
+            return num > T(0) && !isnan(st) ? st : T(0);
         }
     } else {
         if constexpr (LIM == LIM_SUPERBEE) {
