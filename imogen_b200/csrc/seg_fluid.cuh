@@ -469,8 +469,9 @@ __device__ __forceinline__ void sp_sync(const SweepGeom& g) {
 
 // ---- predictor and corrector of one lane of variables --------------------------------------------------
 // Which of a segment's cells round the change of the half step before they add it (FluidArgs.round_cells = n: a
-// pencil's cells n - 1, 2 n - 1, ..., the energy excepted): END the last one, MID the fourth of 8; 0 none, 1 yes, 2 as
-// the launch says (round_cells is 4 in form 1 of the MHD fluxes wherever C is a multiple of 4, and 0 in form 2).
+// pencil's cells n - 1, 2 n - 1, ..., the energy excepted), among the last one and the fourth of 8 (any of 3): 0 none,
+// 1 yes, 2 as the launch says (round_cells is 4 in form 1 of the MHD fluxes wherever C is a multiple of 4, and 0 in
+// form 2).
 template <typename T, int MHD, int C>
 __host__ __device__ constexpr int seg_round_mode() {
     return sizeof(T) == 8 || MHD == 2 ? 0 : (MHD == 1 && C % 4 == 0 ? 1 : 2);
@@ -478,8 +479,8 @@ __host__ __device__ constexpr int seg_round_mode() {
 
 // Predictor (relaxingFluid.m:30-39): u and F at cells -1 .. C (index j + 1); ic = 1 / c_f, h = dt/dx c_f / 4.
 template <typename V, int C, int RND>
-__device__ __forceinline__ void seg_predict(const V (&u)[C + 2], const V (&F)[C + 2], V ic, V nic, V h, V nh, bool round4,
-                                            bool round_end, V (&us)[C]) {
+__device__ __forceinline__ void seg_predict(const V (&u)[C + 2], const V (&F)[C + 2], V ic, V nic, V h, V nh, unsigned round,
+                                            V (&us)[C]) {
     V R[C + 1], L[C + 1];   // 2R at cells -1 .. C-1 (j + 1), 2L at cells 0 .. C (j)
 #pragma unroll
     for (int j = 0; j <= C; ++j) {
@@ -494,8 +495,8 @@ __device__ __forceinline__ void seg_predict(const V (&u)[C + 2], const V (&F)[C 
             us[k] = v_sub(u[k + 1], v_mul(h, S));
         } else {
             us[k] = v_fma(nh, S, u[k + 1]);
-            if (RND == 2 && (k == C - 1 || k % 4 == 3))
-                us[k] = v_pick(k == C - 1 ? round_end : round4, v_sub(u[k + 1], v_mul(h, S)), us[k]);
+            if (RND == 2 && (C == 3 || k == C - 1 || k % 4 == 3))
+                us[k] = v_pick(round >> k & 1, v_sub(u[k + 1], v_mul(h, S)), us[k]);
         }
     }
 }
@@ -560,7 +561,7 @@ __device__ __forceinline__ bool is_cell(int k, int n) {
 }
 // What the stages need to know of a thread's place: its neighbours' records, the ends it sits at, its own cells.
 struct SegEnds {
-    bool round4, round_end;   // seg_predict
+    unsigned round;          // seg_predict: the cells that round (bit k)
     SegRef l1, l2, r1, r2;   // cells -1, -2 and the two past the last own cell
     bool circ_lo, circ_hi;
     bool solo;               // the whole pencil in this thread: its neighbours are its own cells
@@ -601,7 +602,7 @@ __device__ __forceinline__ void seg_predict_vars(const SegEnds& e, T (&u)[5][C],
             f[k + 1] = v_pick(here, f[C + 1], f[k + 1]);
         }
     }
-    seg_predict<V, C, v < 4 ? RND : 0>(a, f, v_dup<V>(ic), v_dup<V>(-ic), v_dup<V>(qh), v_dup<V>(-qh), e.round4, e.round_end, o);
+    seg_predict<V, C, v < 4 ? RND : 0>(a, f, v_dup<V>(ic), v_dup<V>(-ic), v_dup<V>(qh), v_dup<V>(-qh), e.round, o);
 #pragma unroll
     for (int k = 0; k < C; ++k) L::put(o[k], u[v][k], u[w][k]);
 }
@@ -754,8 +755,11 @@ __device__ __forceinline__ void fluid_seg_body(const FluidArgs& a, unsigned vblo
     const bool lo_own = s == 0 && !circ_lo, hi_own = s == S - 1 && !circ_hi;
     e.lo_own = lo_own;
     const bool tile = sizeof(T) == 4 && a.round_cells == 0;
-    e.round4 = a.round_cells == 4;
-    e.round_end = a.round_cells && (r0 + C) % a.round_cells == 0;
+    e.round = 0;
+    if (sizeof(T) == 4 && a.round_cells)
+#pragma unroll
+        for (int k = 0; k < C; ++k)
+            if (C == 3 || k == C - 1 || k % 4 == 3) e.round |= (unsigned)((r0 + k + 1) % a.round_cells == 0) << k;
     e.hi_own = hi_own;
     SegRef &rl1 = e.l1, &rl2 = e.l2, &rr1 = e.r1, &rr2 = e.r2;
     int lt, rt;                  // threads of the neighbour segments (viscosity: whole segments, one CTA)

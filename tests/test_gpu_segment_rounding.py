@@ -2,12 +2,17 @@
 last bit by several powers of ten in a hundred iterations, so a kernel that replaces another on the same grid has to
 round as it did: one sweep of the segment kernels equals one of the pencil-tile kernels (IMOGEN_B200_TILE_KERNELS=1)
 bit for bit."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 from imogen_b200 import ImogenRun
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 F32 = lambda a: np.asarray(a, dtype=np.float32).astype(np.float64)
 
 
@@ -73,3 +78,72 @@ def test_fade_ends_round_as_in_the_tile_kernels(grid, bc, X, magnet, monkeypatch
     s = _settings(grid, bc, magnet)
     a, b = (_sweep(s, _ordinary(grid, magnet, 5), X, 1e-3, tile, monkeypatch) for tile in (False, True))
     assert all((x == y).all() for x, y in zip(a, b)), [int((x != y).sum()) for x, y in zip(a, b)]
+
+
+def _tilings(n, d, precision="mixed"):
+    """Segment tilings of a pencil of n cells along dimension d, one CTA of at least 64 threads, for each number of cells
+    a thread that may hold (of 3-cell pencils, 3)."""
+    out = []
+    for c in (2, 3, 4, 8):
+        if c == 3 and n % 3 or n == 3 and c != 3:
+            continue
+        s = -(-n // c)
+        for wb in (1, 2, 4, 8, 16, 32) if d == 1 else (4, 8, 16, 32):
+            nt = -(-wb * s // 32) * 32
+            if 64 <= nt <= 512:
+                out.append((wb, s, 1, nt, c, 1, 1))
+                break
+    return out
+
+
+FORMS = [((384, 24, 1), 1), ((24, 48, 1), 2), ((75, 24, 1), 1), ((24, 90, 1), 2), ((24, 24, 51), 3)]
+
+
+def _tiled_sweep(grid, X, magnet, tiling=None, tune=False):
+    r = ImogenRun(precision="mixed", **_settings(grid, "circ", magnet))
+    st = _ordinary(grid, magnet, 3)(None)
+    r.set_state(*st)
+    if tune:
+        r.autotune(1)
+        r.set_state(*st)
+    if tiling:
+        r.set_tiling(X, tiling)
+    used = r.tiling("fluid")[X]
+    r.time.set(0.0, 0.0, 1)
+    r.relaxing_fluid(2 if X == 1 else 1)
+    r.time.set(0.0, 1e-3, 1)
+    r.relaxing_fluid(X)
+    out = [r.download(k) for k in ("mass", "momx", "momy", "momz", "ener")]
+    r.close()
+    return used, out
+
+
+def _same(a, b):
+    return all((x == y).all() for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("magnet", [False, True])
+@pytest.mark.parametrize("grid,X", FORMS)
+def test_any_segment_tiling_rounds_alike(grid, X, magnet):
+    """Grids of either form of the fluxes (whole 4-cell segments that fill CTAs, or not): the default tiling, the same
+    one picked and every other number of cells a thread give the same bits."""
+    default, want = _tiled_sweep(grid, X, magnet)
+    assert default[6]
+    tried = _tilings(grid[X - 1], X)
+    assert len({t[4] for t in tried}) >= 3
+    for t in [default, *tried]:
+        assert _same(want, _tiled_sweep(grid, X, magnet, t)[1]), t
+
+
+def _after_autotuning(grid, X, magnet):
+    default, want = _tiled_sweep(grid, X, magnet)
+    assert _same(want, _tiled_sweep(grid, X, magnet, default, tune=True)[1])
+    assert _same(want, _tiled_sweep(grid, X, magnet, default)[1])   # created with what the other one's autotuning picked
+
+
+def test_autotuning_leaves_the_rounding():
+    """In a process of its own: what the autotuner picks serves every later run of the process."""
+    code = "from tests.test_gpu_segment_rounding import *\nfrom tests.test_gpu_segment_rounding import _after_autotuning\n" \
+           "for grid, X in FORMS:\n    for magnet in (False, True):\n        _after_autotuning(grid, X, magnet)\n"
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
