@@ -730,7 +730,8 @@ __device__ __forceinline__ void fluid_seg_body(const FluidArgs& a, unsigned vblo
     __shared__ double cflp[3][MAX_WARPS];
     using U = typename SegBits<T>::U;
     const SweepGeom& g = a.sg;
-    const int NT = g.NT, S = g.G, d = g.d, d1 = g.d1, d2 = g.d2, N = g.N;
+    // (a batch may launch a member's CTAs with more threads than its tiling has: they idle)
+    const int NT = CLU ? g.NT : (int)blockDim.x, S = g.G, d = g.d, d1 = g.d1, d2 = g.d2, N = g.N;
     const int t = threadIdx.x;
     SegPos sp;
     sp.init<CLU>(g, vblock);

@@ -278,7 +278,7 @@ __device__ __forceinline__ void mag_chain_win_body(const MagArgs& a, unsigned vb
     using Rec = ChainRec<V>;
     constexpr int PASSES = ChainLane<T>::PASSES;
     const SweepGeom& g = a.sg;
-    const int N = g.N, S = g.G, NT = g.NT, d = g.d;
+    const int N = g.N, S = g.G, NT = g.CL > 1 ? g.NT : (int)blockDim.x, d = g.d;   // (blockDim: as in the fluid kernels)
     WinPos wp;
     wp.init(g, vblock);
     const int r0 = wp.s * C;
