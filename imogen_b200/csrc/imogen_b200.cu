@@ -184,6 +184,8 @@ struct img_ctx {
     int iters_base = 0;
     PencilCfg pcfg[3][3];        // pencil tiling per kernel (0 fluid sweep, 1 magnet chain, 2 magnet CT) and
                                  // direction; the public magnet tiling sets 1 and 2, the autotuner tunes 2 alone
+    PencilCfg pcfg_full[3];      // fluid sweep per direction: as a member of a batch that fills the chip
+    bool full = false;           // recording for such a batch
     PencilCfg pcfg_tile[3];      // fluid sweep per direction: the tile-kernel tiling of the launches that the
                                  // segment kernel does not take (stored-edge capture, fade, other ends)
     PencilCfg pcfg_mtile[2][3];  // the same for the magnet chain [0] and CT pass [1] (window kernels)
@@ -557,7 +559,8 @@ const PencilCfg* default_segments(const std::vector<PencilCfg>& c, const Geom& g
 // of work is what takes the time, and 2 cells a thread in CTAs of 128 make the faster fluid sweeps (one iteration: 64^2
 // mixed 53 -> 45 us, 64^2 FP64 89 -> 75 us, 24^3 mixed 78 -> 68 us; 200^2 60 -> 57 us; 512^2 is past the line: x fluid
 // sweep 7.5 us with 4 cells, 9.2 us with 2).
-bool small_grid(const Geom& g) { return g.ncell < 4 * 148 * 256; }
+constexpr long long kFullCells = 4 * 148 * 256;
+bool small_grid(const Geom& g) { return g.ncell < kFullCells; }
 
 // Default magnet tiling: the window kernels where a default window tiling exists, else the tile kernels'
 // default.  4 cells a thread and CTAs of 256 threads (512 share an SM by two as well: rows of 32 bytes come
@@ -574,12 +577,13 @@ PencilCfg choose_window(const Geom& g, int d, size_t elem, const PencilCfg& tile
 // 256, 425 with 512; y 504 us with 4 pencils in 256 threads, 534 with 8 in 512).  FP64: 2 cells a thread while two CTAs'
 // exchange records fit an SM (192 threads; 96^3 x 50 us, y 57 us), else 4 (96^3: 62 and 65 us; 128^3 y: 137 us,
 // with 2 cells in 256 threads 199 us).
-PencilCfg choose_fluid(const Geom& g, int d, size_t elem, const PencilCfg& tile) {
+// `full`: beside other grids of a batch that fill the chip together.
+PencilCfg choose_fluid(const Geom& g, int d, size_t elem, const PencilCfg& tile, bool full) {
     std::vector<PencilCfg> c = seg_candidates(g, d, elem);   // with room for the anchors of fade ends
     c.erase(std::remove_if(c.begin(), c.end(),
                            [&](const PencilCfg& p) { return seg_smem(elem, p.NT, p.Wb, false, p.CL == 1) > kPencilSmemLimit; }), c.end());
     // (longer pencils keep 4: their CTAs have the warps, and tubes of an ensemble fill the chip together)
-    const PencilCfg* best = small_grid(g) && g.n[d] <= 256 ? default_segments(c, g, d, elem, 2, 128, 2.0) : nullptr;
+    const PencilCfg* best = !full && small_grid(g) && g.n[d] <= 256 ? default_segments(c, g, d, elem, 2, 128, 2.0) : nullptr;
     if (!best && elem == 8) {
         std::vector<PencilCfg> two;
         for (const PencilCfg& p : c)
@@ -779,7 +783,7 @@ int launch_fluid(img_ctx* ctx, int d, bool cfl) {
     // run's first sweep) and other ends take the tile kernels
     const bool fade = fade_on(c, d, CLS_MASS, CLS_ENER);
     const bool init = ctx->init_store || ctx->init_flux;
-    const PencilCfg& ps = ctx->pcfg[0][d];
+    const PencilCfg& ps = ctx->full ? ctx->pcfg_full[d] : ctx->pcfg[0][d];
     bool seg_ok = ps.seg && !init &&
                   !(fade && (ps.CL > 1 || (ps.seg != 2 && ps.seg != 4) || seg_smem(sizeof(T), ps.NT, ps.Wb, false, true) > kPencilSmemLimit));
     for (int k = 0; k < 3; ++k)
@@ -789,7 +793,7 @@ int launch_fluid(img_ctx* ctx, int d, bool cfl) {
     // (img_create and img_set_tiling see to it), so no stored edge is ever read: the first sweeps too
     const bool visc = c.viscosity_type != IMG_VISC_NONE;
     if (visc) seg_ok = true;
-    const PencilCfg& pcf = (seg_ok || !ctx->pcfg[0][d].seg) ? ctx->pcfg[0][d] : ctx->pcfg_tile[d];
+    const PencilCfg& pcf = (seg_ok || !ps.seg) ? ps : ctx->pcfg_tile[d];
     a.sg = sweep_geom(ctx, d, pcf);
     for (int v = 0; v < NQ; ++v) a.q[v] = ctx->q[v];
     a.tm = ctx->tm;
@@ -1462,7 +1466,7 @@ int img_create(img_ctx** out, const img_config* cfg) {
             if (kind == 0) {
                 ctx->pcfg_tile[d] = ctx->pcfg[0][d];
                 if (tile_only) continue;
-                ctx->pcfg[0][d] = choose_fluid(g, d, ctx->elem, ctx->pcfg_tile[d]);
+                ctx->pcfg[0][d] = choose_fluid(g, d, ctx->elem, ctx->pcfg_tile[d], false);
             } else {
                 ctx->pcfg_mtile[kind - 1][d] = ctx->pcfg[kind][d];
                 if (tile_only) continue;
@@ -1482,6 +1486,11 @@ int img_create(img_ctx** out, const img_config* cfg) {
             std::lock_guard<std::mutex> lock(g_tune_mu);
             auto it = g_tuned.find(tune_key(kind, g, d, ctx->elem, *cfg));
             if (it != g_tuned.end()) ctx->pcfg[kind][d] = it->second;
+            if (kind == 0) {
+                ctx->pcfg_full[d] = ctx->pcfg[0][d];
+                const PencilCfg f = choose_fluid(g, d, ctx->elem, ctx->pcfg_tile[d], true);
+                if (it == g_tuned.end() && !tile_only && f.seg) ctx->pcfg_full[d] = f;   // (the same kernel family)
+            }
         }
 
     auto bail = [&](int code) {
@@ -2609,11 +2618,16 @@ int img_batch_step(img_batch* b) {
         return IMG_OK;
     }
     std::vector<std::vector<OpRec>> recs(b->members.size());
+    long long cells = 0;
+    for (const img_ctx* m : b->members) cells += m->g.ncell;
+    const bool full = cells >= kFullCells;   // no member is small beside the others
     for (size_t i = 0; i < b->members.size(); ++i) {
         img_ctx* m = b->members[i];
+        m->full = full;
         m->rec = &recs[i];
         int rc = enqueue_iteration(m);
         m->rec = nullptr;
+        m->full = false;
         if (rc != IMG_OK) return bfail(b, rc, "member %zu: %s", i, m->err.c_str());
     }
     // a steady plan is kept (and captured as a graph) from the second cycle of a membership on,
@@ -2882,6 +2896,7 @@ int img_autotune(img_ctx* ctx, int trials) {
                 }
             }
             ctx->pcfg[kind][d] = best;
+            if (kind == 0) ctx->pcfg_full[d] = best;
             std::lock_guard<std::mutex> lock(g_tune_mu);
             g_tuned[tune_key(kind, ctx->g, d, ctx->elem, ctx->cfg)] = best;
         }
@@ -2915,6 +2930,7 @@ int img_set_tiling(img_ctx* ctx, int dim, const int cfg[7]) {
         c.nqc = nqc;
         if (c.seg) {
             ctx->pcfg[kind][d] = c;
+            if (kind == 0) ctx->pcfg_full[d] = c;
             if (kind == 1) ctx->pcfg[2][d] = c;
             drop_graphs(ctx);
             return IMG_OK;
@@ -2928,6 +2944,7 @@ int img_set_tiling(img_ctx* ctx, int dim, const int cfg[7]) {
             return fail(ctx, IMG_ERR_UNSUPPORTED, "tiling cannot be scheduled on this device");
         }
         ctx->pcfg[kind][d] = c;
+        if (kind == 0) ctx->pcfg_full[d] = c;
         if (kind == 1) ctx->pcfg[2][d] = c;   // the public magnet tiling is the chain's and the CT's
         drop_graphs(ctx);
         return IMG_OK;
