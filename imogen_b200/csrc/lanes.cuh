@@ -41,12 +41,9 @@ template <typename T> __device__ __forceinline__ T v_pick(bool c, T a, T b) { re
 
 // The limiter correction of each lane.  Van Leer: dL dR / (dL + dR) where the product is positive, else 0.
 // A positive FP32 product keeps |dL + dR| above 2^-75, so the one-instruction reciprocal never sees a
-// subnormal (which its .ftz form would flush).
-// Where both overflow the quotient is inf * 0 and the correction 0, as in limiter_corr_t.
-__device__ __forceinline__ float vanleer_part(float p, float s) {
-    const float q = p * rcp_ftz(s);
-    return p > 0.f && q == q ? q : 0.f;
-}
+// subnormal (which its .ftz form would flush).  The maximum with 0 takes negative products and NaN (both
+// overflow: inf * 0), as limiter_corr_t does; the sign of the sum follows.
+__device__ __forceinline__ float vanleer_part(float p, float s) { return copysignf(fmaxf(p * rcp_ftz(fabsf(s)), 0.f), s); }
 template <int LIM>
 __device__ __forceinline__ float v_limit(float dL, float dR) {
     if constexpr (LIM == LIM_VANLEER) return vanleer_part(dL * dR, dL + dR);
