@@ -49,6 +49,7 @@ struct PencilCfg {
     int Wb = 1, G = 32, CL = 1, NT = 32, cpt = 2;
     int nqc = 1;   // magnet chain: transverse components per CTA
     int seg = 0;   // fluid sweep: segment kernel with seg = cpt consecutive cells per thread (G = N / cpt)
+    bool picked = false;   // by the autotuner or img_set_tiling, not a default
 };
 
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -750,16 +751,17 @@ PencilLaunch pencil_launch(const img_ctx* ctx, const PencilCfg& pcf, int d, size
 
 // The rounding of a segment launch (FP32; FP64 has form 1 alone).  Form 2 rounds every sum as the pencil-tile
 // kernels do, form 1 differs from it in the last bit of the fluxes' B terms and of every fourth cell's half step
-// (seg_flux, seg_predict).  A grid's steps have to keep rounding alike, for FP32 differences grow with the flow's own
-// instabilities (a 64^2 vortex: from the last bit to 2e-5 in 60 steps, 256^3 shear layers past 1e-3 in 120), so the form
-// follows the grid, not the tiling: any segment tiling of a grid gives the same bits (of
-// 3-cell pencils, those of 3 cells a thread).  Form 1: artificial viscosity;
-// pencils of whole 4-cell segments that make CTAs of 64 to 512 threads (x: a power of two up to 32 of them or a multiple of 32, or 64 and
-// more with const ends; y and z: 8 pencils side by side); whole pencils of one thread across y and z.  Form 2: the
-// others, which the tile kernels can serve too.
-int flux_form(const Geom& g, int d, size_t elem, const img_config& c, bool fade) {
+// (seg_flux, seg_predict).  FP32 differences grow with the flow's own instabilities (a 64^2 vortex: from the last bit to
+// 2e-5 in 60 steps, 256^3 shear layers past 1e-3 in 120), so what a run has always given, it keeps: a grid whose default
+// was a tile kernel keeps that one's rounding (form 2) under its default tiling, and a segment tiling that the
+// autotuner or img_set_tiling picks has form 1 on every grid.  So the bits depend on whether the tiling is the default
+// or a picked one (a picked tiling serves the process's later runs of the same key too), but not on which segment
+// tiling it is (of 3-cell pencils: of 3 cells a thread), nor on batching.  Form 1 by default: artificial viscosity; pencils
+// of whole 4-cell segments that make CTAs of 64 to 512 threads (x: a power of two up to 32 of them or a multiple of 32,
+// or 64 and more with const ends; y and z: 8 pencils side by side); whole pencils of one thread across y and z.
+int flux_form(const Geom& g, int d, size_t elem, const img_config& c, bool fade, bool picked) {
     if (fade) return 2;
-    if (elem == 8 || c.viscosity_type != IMG_VISC_NONE) return 1;
+    if (elem == 8 || picked || c.viscosity_type != IMG_VISC_NONE) return 1;
     const int N = g.n[d], S = (N + 3) / 4;
     const long long ncol = g.ncell / N;
     const bool fits_x = S % 32 == 0 || (S <= 32 && 32 % S == 0);
@@ -841,7 +843,7 @@ int launch_fluid(img_ctx* ctx, int d, bool cfl) {
         }
     L.init = a.init_store || a.init_flux;   // first sweeps: the stored-edge capturing kernel
     if (L.seg) L.cg = true;                  // segment kernels index their ghosts directly
-    const int form = L.seg ? flux_form(ctx->g, d, sizeof(T), c, fade) : 1, mhd = ctx->mhd ? form : 0;
+    const int form = L.seg ? flux_form(ctx->g, d, sizeof(T), c, fade, pcf.picked) : 1, mhd = ctx->mhd ? form : 0;
     a.round_cells = sizeof(T) == 4 && form == 1 ? (ctx->g.n[d] < 4 ? ctx->g.n[d] : 4) : 0;
     if (ctx->rec) {
         OpRec r{};
@@ -2895,6 +2897,7 @@ int img_autotune(img_ctx* ctx, int trials) {
                     best = cand;
                 }
             }
+            best.picked = true;
             ctx->pcfg[kind][d] = best;
             if (kind == 0) ctx->pcfg_full[d] = best;
             std::lock_guard<std::mutex> lock(g_tune_mu);
@@ -2928,6 +2931,7 @@ int img_set_tiling(img_ctx* ctx, int dim, const int cfg[7]) {
             (c.seg != 0) != (cfg[6] != 0))
             continue;
         c.nqc = nqc;
+        c.picked = true;
         if (c.seg) {
             ctx->pcfg[kind][d] = c;
             if (kind == 0) ctx->pcfg_full[d] = c;

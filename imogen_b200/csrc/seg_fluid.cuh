@@ -24,8 +24,9 @@
 // behind one more barrier: four barriers instead of two.
 // Per cell the operations are those of the pencil-tile kernels (fluid_sweep.cuh) in the same order; the momentum
 // and cell-centred B are held in sweep-rotated order (the component along the sweep first).  The FMAs are written
-// out (the unit is compiled without implicit ones), so results do not depend on the tiling.  MHD = 2 sums and
-// rounds the B terms of the fluxes as the pencil-tile kernels do, MHD = 1 in rotated order (seg_flux).
+// out (the unit is compiled without implicit ones), so within one form of the fluxes results do not depend on the
+// tiling.  MHD = 2 sums and rounds the B terms of the fluxes as the pencil-tile kernels do, MHD = 1 in rotated order
+// (seg_flux); the launch picks the form.
 //
 // Thread placement (SweepGeom with G = S segments per pencil, RC = N): along x the S threads of a
 // pencil are consecutive (thread t = b*S + s), along y and z the Wb pencils of the CTA are (t = s*Wb +
