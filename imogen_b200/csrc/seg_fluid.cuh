@@ -165,20 +165,20 @@ __device__ __forceinline__ void win_store(void* ptr, int o, int sd, bool vec, in
 
 // Constants of the 'totsnd' pressure (pressure.m:23-64) from gamma.
 struct SegPressure {
-    double g, g1, half_g1, p_ms;
-    __device__ __forceinline__ explicit SegPressure(double G) : g(G), g1(G - 1.0), half_g1((G - 1.0) * 0.5), p_ms(0.5 * (2.0 - G)) {}
-    // P and rho c_s^2 from x = E - rho v^2/2 and msq = B^2.  Each B^2 term is rounded before it joins (G-1) x, as
+    double half_g, g1, half_g1, p_ms;
+    __device__ __forceinline__ explicit SegPressure(double G) : half_g(0.5 * G), g1(G - 1.0), half_g1((G - 1.0) * 0.5), p_ms(0.5 * (2.0 - G)) {}
+    // P and rho c_s^2 / 2 from x = E - rho v^2/2 and msq = B^2.  Each B^2 term is rounded before it joins (G-1) x, as
     // the pencil-tile kernels' pressure_totsnd_mixed comes out, whose FP64 bits the mixed form shares: one of the
     // other orders differs in the last FP64 bit of every other cell, hence in the FP32 pressure of one in 2e9, and a
     // 256^3 shear run grows that to 1e-3 of B's scale at single cells in 120 iterations.
     template <int MSQ>
-    __device__ __forceinline__ void totals(double x, double msq, double& pt, double& c2) const {
+    __device__ __forceinline__ void totals(double x, double msq, double& pt, double& hc2) const {
         if constexpr (MSQ) {
-            c2 = fma(g, fma(g1, x, -(half_g1 * msq)), 2.0 * msq);
+            hc2 = fma(half_g, fma(g1, x, -(half_g1 * msq)), msq);
             pt = fma(g1, x, p_ms * msq);
         } else {
             pt = g1 * x;
-            c2 = g * pt;
+            hc2 = half_g * pt;
         }
     }
 };
@@ -195,9 +195,9 @@ __device__ __forceinline__ float seg_pressure(const SegPressure& k, const float 
     const double inv = e0 * fma(-(double)u[0], e0, 2.0);
     const double px = u[1], py = u[2], pz = u[3];
     const double psq = fma(pz, pz, fma(px, px, py * py));
-    double c2, pt;
-    k.totals<MSQ>(fma(-(0.5 * psq), inv, (double)u[4]), msq, pt, c2);
-    cs = sqrt_approx(fabsf((float)(c2 * inv)));
+    double hc2, pt;
+    k.totals<MSQ>(fma(-(0.5 * psq), inv, (double)u[4]), msq, pt, hc2);
+    cs = sqrt_approx(fabsf(2.f * (float)(hc2 * inv)));
     p = pt < 0 ? 0.f : (float)pt;
     return fabsf(u[1] * ir) + cs;
 }
@@ -206,9 +206,9 @@ __device__ __forceinline__ double seg_pressure(const SegPressure& k, const doubl
                                                double& ir) {
     ir = recip(u[0]);
     const double psq = fma(u[3], u[3], fma(u[1], u[1], u[2] * u[2]));
-    double c2, pt;
-    k.totals<MSQ>(fma(-(0.5 * psq), ir, u[4]), msq, pt, c2);
-    cs = sqrt_goldschmidt(fabs(c2 * ir));
+    double hc2, pt;
+    k.totals<MSQ>(fma(-(0.5 * psq), ir, u[4]), msq, pt, hc2);
+    cs = sqrt_goldschmidt(fabs(2.0 * (hc2 * ir)));
     p = pt < 0 ? 0.0 : pt;
     return fabs(u[1] * ir) + cs;
 }
