@@ -19,7 +19,10 @@ void (*fluid_seg_kernel_c(int C))(const FluidArgs) {
     if constexpr (!CLU && !FADE) {
         if (C == 3) return fluid_seg_kernel<T, MHD, 3, VISC_NONE, CLU, FADE, MAXT>;
     }
-    return C == 2 ? fluid_seg_kernel<T, MHD, 2, VISC_NONE, CLU, FADE, MAXT> : fluid_seg_kernel<T, MHD, 4, VISC_NONE, CLU, FADE, MAXT>;
+    if constexpr (MAXT > 256) {
+        if (C == 2) return fluid_seg_kernel<T, MHD, 2, VISC_NONE, CLU, FADE, MAXT>;
+    }
+    return fluid_seg_kernel<T, MHD, 4, VISC_NONE, CLU, FADE, MAXT>;
 }
 
 template <typename T, int MHD, bool CLU, bool FADE, int MAXT>
@@ -30,13 +33,19 @@ void (*fluid_seg_batch_kernel_c(int C))(const FluidArgs*, const BlockMap*) {
     if constexpr (!CLU && !FADE) {
         if (C == 3) return fluid_seg_batch_kernel<T, MHD, 3, CLU, FADE, MAXT>;
     }
-    return C == 2 ? fluid_seg_batch_kernel<T, MHD, 2, CLU, FADE, MAXT> : fluid_seg_batch_kernel<T, MHD, 4, CLU, FADE, MAXT>;
+    if constexpr (MAXT > 256) {
+        if (C == 2) return fluid_seg_batch_kernel<T, MHD, 2, CLU, FADE, MAXT>;
+    }
+    return fluid_seg_batch_kernel<T, MHD, 4, CLU, FADE, MAXT>;
 }
 
 // With artificial viscosity: 2 and 4 cells per thread.
 template <typename T, int MHD, int VT, int MAXT>
 void (*fluid_seg_visc_kernel_c(int C))(const FluidArgs) {
-    return C == 2 ? fluid_seg_kernel<T, MHD, 2, VT, false, false, MAXT> : fluid_seg_kernel<T, MHD, 4, VT, false, false, MAXT>;
+    if constexpr (MAXT > 256) {
+        if (C == 2) return fluid_seg_kernel<T, MHD, 2, VT, false, false, MAXT>;
+    }
+    return fluid_seg_kernel<T, MHD, 4, VT, false, false, MAXT>;
 }
 
 // Forms of the MHD fluxes (seg_flux): fade ends take form 2, artificial viscosity form 1, FP64 otherwise form 1 and
@@ -102,6 +111,7 @@ cudaError_t fluid_seg_attributes(int optin) {
             for (int form = 0; form < 3; ++form) {   // plain, over a cluster, with fade ends
                 if ((form == 1 && C == 3) || (form == 2 && C != 2 && C != 4)) continue;
                 for (unsigned block : {256u, 512u}) {
+                    if (block == 256 && (sizeof(T) == 4 || C == 2)) continue;   // the same kernels as 512's
                     cudaError_t e = allow_max_smem(fluid_seg_kernel_p<T>(C, mhd, form == 1, form == 2, VISC_NONE, block), optin);
                     if (e == cudaSuccess)
                         e = allow_max_smem(fluid_seg_batch_kernel_p<T>(C, mhd, form == 1, form == 2, block), optin);
