@@ -490,8 +490,9 @@ std::vector<PencilCfg> seg_candidates(const Geom& g, int d, size_t elem, bool vi
 // cells per thread, S = ceil(N / C) threads per pencil (the last segment may be shorter), whole pencils in one
 // CTA of NT = Wb * S threads rounded up to a multiple of 32 (32 <= NT <= 512, the threads past the segments
 // idle); along y and z Wb >= 4 pencils side by side (2 where 4 do not fit; up to 64, or to the CTA where each
-// pencil is one thread's), along x up to 64, or to the CTA where the last segment is shorter.  Along x, for S above 256 (512) segments, one pencil over a cluster of
-// CL = ceil(S / 256) <= 8 CTAs (ceil(S / 512) <= 4) of NT = ceil(S / CL) rounded up.
+// pencil is one thread's), along x up to 64, or to the CTA where the last segment is shorter.  Along x, for S above
+// 256 (512) segments, one pencil over a cluster of CL = ceil(S / 256) <= 8 CTAs (ceil(S / 512) <= 4) of
+// NT = ceil(S / CL) rounded up.
 std::vector<PencilCfg> win_candidates(const Geom& g, int d) {
     std::vector<PencilCfg> out;
     const int N = g.n[d];
@@ -574,7 +575,7 @@ PencilCfg choose_window(const Geom& g, int d, size_t elem, const PencilCfg& tile
 
 // Default fluid tiling: the segment kernel where a default segment tiling exists, else the tile kernels'
 // default.  Mixed: 4 cells a thread, CTAs of 128 threads along x and 256 along y and z; one of 512 has an SM to
-// itself and nothing to hide its barriers behind (256^3, at the time: x 324 us with 64 to 128 threads, 355 with
+// itself and nothing to hide its barriers behind (256^3, an earlier build: x 324 us with 64 to 128 threads, 355 with
 // 256, 425 with 512; y 504 us with 4 pencils in 256 threads, 534 with 8 in 512).  FP64: 2 cells a thread while two CTAs'
 // exchange records fit an SM (192 threads; 96^3 x 50 us, y 57 us), else 4 (96^3: 62 and 65 us; 128^3 y: 137 us,
 // with 2 cells in 256 threads 199 us).
@@ -787,7 +788,8 @@ int launch_fluid(img_ctx* ctx, int d, bool cfl) {
     const bool init = ctx->init_store || ctx->init_flux;
     const PencilCfg& ps = ctx->full ? ctx->pcfg_full[d] : ctx->pcfg[0][d];
     bool seg_ok = ps.seg && !init &&
-                  !(fade && (ps.CL > 1 || (ps.seg != 2 && ps.seg != 4) || seg_smem(sizeof(T), ps.NT, ps.Wb, false, true) > kPencilSmemLimit));
+                  !(fade && (ps.CL > 1 || (ps.seg != 2 && ps.seg != 4) ||
+                             seg_smem(sizeof(T), ps.NT, ps.Wb, false, true) > kPencilSmemLimit));
     for (int k = 0; k < 3; ++k)
         for (int side = 0; side < 2; ++side)
             if (!copy_ghost_mode(c.bc_modes[k][side][d]) || c.bc_modes[k][side][d] != c.bc_modes[CLS_MASS][side][d]) seg_ok = false;
@@ -2352,8 +2354,10 @@ bool join_shape(PencilLaunch& x, const PencilLaunch& y, int kind, size_t elem) {
     PencilLaunch w = x;
     w.block = std::max(x.block, y.block);
     w.pencils = std::max(x.pencils, y.pencils);
-    w.smem = kind == OP_FLUID ? seg_smem(elem, w.block, w.pencils, false, w.fade)
-                              : (kind == OP_CHAIN ? (elem == 8 ? chain_win_smem_bytes<double>(w.block, w.seg) : chain_win_smem_bytes<float>(w.block, w.seg)) : 0);
+    w.smem = 0;
+    if (kind == OP_FLUID) w.smem = seg_smem(elem, w.block, w.pencils, false, w.fade);
+    else if (kind == OP_CHAIN)
+        w.smem = elem == 8 ? chain_win_smem_bytes<double>(w.block, w.seg) : chain_win_smem_bytes<float>(w.block, w.seg);
     if (w.smem > kPencilSmemLimit) return false;
     x = w;
     return true;

@@ -14,8 +14,8 @@
 //            (relaxingFluid.m:57-62) -- the limited values of the neighbour cells next to the segment are
 //            computed here as well, from the published cells -- and the update (relaxingFluid.m:64-71);
 //            store; fused CFL maxima on the last sweep of a step.
-// R = (u + F/c_f)/2 and L = (u - F/c_f)/2 take one FMA each (the predictor leaves the 2 to the update).  In the mixed form two variables at a time go through the
-// packed FP32 instructions (lanes.cuh).
+// R = (u + F/c_f)/2 and L = (u - F/c_f)/2 take one FMA each (the predictor leaves the 2 to the update).  In the mixed
+// form two variables at a time go through the packed FP32 instructions (lanes.cuh).
 // Fade ends (fade_shift.m) blend every shifted array near the ends toward the shifted end values: those
 // launches (FADE) form the shifted values cell by cell, take the ends' rows from a small anchor set and
 // exchange the limited fluxes behind one more barrier.
@@ -166,7 +166,8 @@ __device__ __forceinline__ void win_store(void* ptr, int o, int sd, bool vec, in
 // Constants of the 'totsnd' pressure (pressure.m:23-64) from gamma.
 struct SegPressure {
     double half_g, g1, half_g1, p_ms;
-    __device__ __forceinline__ explicit SegPressure(double G) : half_g(0.5 * G), g1(G - 1.0), half_g1((G - 1.0) * 0.5), p_ms(0.5 * (2.0 - G)) {}
+    __device__ __forceinline__ explicit SegPressure(double G)
+        : half_g(0.5 * G), g1(G - 1.0), half_g1((G - 1.0) * 0.5), p_ms(0.5 * (2.0 - G)) {}
     // P and rho c_s^2 / 2 from x = E - rho v^2/2 and msq = B^2.  Each B^2 term is rounded before it joins (G-1) x, as
     // the pencil-tile kernels' pressure_totsnd_mixed comes out, whose FP64 bits the mixed form shares: one of the
     // other orders differs in the last FP64 bit of every other cell, hence in the FP32 pressure of one in 2e9, and a
@@ -659,7 +660,8 @@ __device__ __forceinline__ void seg_correct_vars(const SegEnds& e, const T (&u)[
     for (int k = 0; k < C; ++k) a[k] = L::get(u[v][k], u[w][k]);
 #pragma unroll
     for (int j = 0; j < C + 4; ++j) x[j] = v_mul(x[j], v_splat<V>(0.5));
-    seg_correct<V, C, LIM>(a, x, f, v_dup<V>(T(0.5) * ics), v_dup<V>(T(-0.5) * ics), v_dup<V>(-ffc), e.lo_own, e.hi_own ? e.nown - 1 : C, o);
+    seg_correct<V, C, LIM>(a, x, f, v_dup<V>(T(0.5) * ics), v_dup<V>(T(-0.5) * ics), v_dup<V>(-ffc), e.lo_own,
+                           e.hi_own ? e.nown - 1 : C, o);
     T p[C], q[C];
 #pragma unroll
     for (int k = 0; k < C; ++k) {
@@ -1181,15 +1183,16 @@ __device__ __forceinline__ void fluid_seg_body(const FluidArgs& a, unsigned vblo
     }
 }
 
-// What bounds it (256^3 mixed, x, 351 us now): warp issue -- the FP64 pressure recovery, the limiters and the
-// fluxes -- beside HBM, whose 872 MB need 131 us at 6.65 TB/s; y and z (532 and 557 us) also wait for their strided rows of
-// 32 bytes.  The tiling that came before (one FP32 lane per instruction, whole-CTA barriers around idle threads, R and
-// L kept apart) took 408, 583 and 584 us; FP64 pencils and fade ends ran on the pencil tiles (96^3 FP64: 72, 112 and
-// 106 us against 51, 61 and 61 us; 96^3 hydrodynamic fade: 77, 103 and 103 us against 49, 51 and 51 us).  At 128 registers 16 warps share an SM; 80
-// registers for 24 warps spill more than they hide (256^3 y 649 -> 704 us), and persistent CTAs that fetch the
-// next bundle with cp.async lose to plain loads (x 345 -> 410 us, y 593 -> 1020 us: 4-byte copies of strided rows).
+// What bounds it (256^3 mixed, x, 343 us): warp issue -- the FP64 pressure recovery, the limiters and the fluxes --
+// beside HBM, whose 872 MB need 135 us at the measured 6.46 TB/s; y and z (523 and 553 us) also wait for their strided
+// rows of 32 bytes.  One FP32 lane per instruction and whole-CTA barriers around idle threads make that 408, 583 and
+// 584 us.  FP64 and fade ends against the pencil tiles: 96^3 FP64 57, 66 and 66 us against 72, 112 and 106; 96^3
+// hydrodynamic with fade ends, mixed, 50, 52 and 52 us against 77, 103 and 103.  At 128 registers 16 warps share an SM;
+// 80 registers for 24 warps spill more than they hide (256^3 y 649 -> 704 us), and persistent CTAs that fetch the next
+// bundle with cp.async lose to plain loads (x 345 -> 410 us, y 593 -> 1020 us: 4-byte copies of strided rows).
 // FP64 kernels of 3 and 4 cells a thread take CTAs of at most 256 threads with all 255 registers a thread can
-// have (MAXT): at 128 they spill.  The others run at 128, 16 warps an SM.
+// have (MAXT): at 128 they spill.  The others run at 128, 16 warps an SM; FP64 CTAs above 256 threads spill and are still
+// faster than the pencil tiles (y fluid sweep of 700^2: 70 us against 127, of 600^2: 61 against 107).
 template <typename T, int MHD, int C, int VT, bool CLU, bool FADE, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) fluid_seg_kernel(const __grid_constant__ FluidArgs a) {
     fluid_seg_body<T, MHD, C, VT, CLU, FADE>(a, blockIdx.x);

@@ -34,8 +34,8 @@ __device__ __forceinline__ int trans_offset(const MagArgs& a, int q, int ie, int
 }
 
 // Global row of window cell j of segment s (rows r0 + j, wrapped for circ, clamped for const ends).
-// The window reaches at most 4 rows past a segment, so a pencil shorter than that wraps more than once
-// (r >= -4 and r < N + C + 4: the loops run at most a few times).
+// The window reaches 2 rows past a segment, so on a pencil shorter than that a row wraps more than once (the loops run
+// at most a few times).
 __host__ __device__ __forceinline__ int win_row_multi(int r, int N, bool circ_lo, bool circ_hi) {
     if (r < 0) {
         if (!circ_lo) return 0;
@@ -52,7 +52,7 @@ __host__ __device__ __forceinline__ int win_row_multi(int r, int N, bool circ_lo
 
 // The same where one wrap suffices: rows r >= -N and r < 2N (a window that reaches H rows past its
 // segment, on a pencil of N >= C + H rows: the last segment starts at row N - 1 at most).  Selects
-// only, no loop.
+// only, no loop; a host-side check of the looping form (the kernels look such rows up rarely enough for the loop).
 __host__ __device__ __forceinline__ int win_row_once(int r, int N, bool circ_lo, bool circ_hi) {
     const int lo = circ_lo ? r + N : 0, hi = circ_hi ? r - N : N - 1;
     return r < 0 ? lo : (r >= N ? hi : r);
@@ -60,8 +60,8 @@ __host__ __device__ __forceinline__ int win_row_once(int r, int N, bool circ_lo,
 
 // Const ends: the window cells of a stage array A (local cells LO .. HI-1 at A[j + OFS]) past the
 // pencil's lower end copy its row 0 (local cell lend = -r0), those past its upper end its last row
-// (local cell hend = N - 1 - r0): the const ghost of every shifted array (constant_shift.m).  A window
-// reaches 4 cells past its segment, so near an end several segments' windows cross it, and the end row
+// (local cell hend = N - 1 - r0): the const ghost of every shifted array (constant_shift.m).  The stages
+// reach 2 cells past a segment, so near an end several segments' windows cross it, and the end row
 // may be a window cell rather than an own one (short segments, a ragged last segment).
 template <typename T, int OFS, int LO, int HI>
 __device__ __forceinline__ void const_fill(T* A, bool circ_lo, bool circ_hi, int lend, int hend) {
@@ -266,8 +266,8 @@ __device__ __forceinline__ double corner_velocity(double pm, double p, double rm
 // (consecutive threads on consecutive 16 bytes, whichever way the sweep runs); after a barrier it reads
 // the two cells on each side from its neighbours' planes, computes wMag of its own cells, publishes that
 // too, and after a second barrier reads wMag of two cells on each side for the limited flux.  The window
-// form before this one re-read and re-divided all C + 8 cells of the chain's stencil from global memory in
-// every thread (380 instructions a cell), which made it instruction-bound.  64 registers a thread leave 32
+// form without exchanges re-reads and re-divides all C + 8 cells of the chain's stencil from global memory in
+// every thread (380 instructions a cell), which makes it instruction-bound.  64 registers a thread leave 32
 // warps an SM; what bounds it now is the latency of its loads, along y and z also their 32-byte rows.
 // Measured, chain and CT pass of one sweep on 256^3 cells in the mixed form: x 450 -> 205 us, y and z
 // 552 -> 355 us; 512^2 (state in L2): y 20 -> 13 us.
