@@ -564,6 +564,9 @@ const PencilCfg* default_segments(const std::vector<PencilCfg>& c, const Geom& g
 constexpr long long kFullCells = 4 * 148 * 256;
 bool small_grid(const Geom& g) { return g.ncell < kFullCells; }
 
+// Whether the fluid sweep along d takes 2 cells a thread for that (longer pencils keep 4: their CTAs have the warps).
+bool few_cells(const Geom& g, int d) { return small_grid(g) && g.n[d] <= 256; }
+
 // Default magnet tiling: the window kernels where a default window tiling exists, else the tile kernels'
 // default.  4 cells a thread and CTAs of 256 threads (512 share an SM by two as well: rows of 32 bytes come
 // first; 256^3 mixed, y: 8 pencils in 512 threads 355 us, 4 in 256 threads 476 us).
@@ -577,15 +580,14 @@ PencilCfg choose_window(const Geom& g, int d, size_t elem, const PencilCfg& tile
 // default.  Mixed: 4 cells a thread, CTAs of 128 threads along x and 256 along y and z; one of 512 has an SM to
 // itself and nothing to hide its barriers behind (256^3, an earlier build: x 324 us with 64 to 128 threads, 355 with
 // 256, 425 with 512; y 504 us with 4 pencils in 256 threads, 534 with 8 in 512).  FP64: 2 cells a thread while two CTAs'
-// exchange records fit an SM (192 threads; 96^3 x 50 us, y 57 us), else 4 (96^3: 62 and 65 us; 128^3 y: 137 us,
-// with 2 cells in 256 threads 199 us).
+// exchange records fit an SM (192 threads; 96^3 x 57 us, y 66 us), else 4 (96^3: 71 and 74 us; 128^3 y: 152 us,
+// with 2 cells in 256 threads 235 us).
 // `full`: beside other grids of a batch that fill the chip together.
 PencilCfg choose_fluid(const Geom& g, int d, size_t elem, const PencilCfg& tile, bool full) {
     std::vector<PencilCfg> c = seg_candidates(g, d, elem);   // with room for the anchors of fade ends
     c.erase(std::remove_if(c.begin(), c.end(),
                            [&](const PencilCfg& p) { return seg_smem(elem, p.NT, p.Wb, false, p.CL == 1) > kPencilSmemLimit; }), c.end());
-    // (longer pencils keep 4: their CTAs have the warps, and tubes of an ensemble fill the chip together)
-    const PencilCfg* best = !full && small_grid(g) && g.n[d] <= 256 ? default_segments(c, g, d, elem, 2, 128, 2.0) : nullptr;
+    const PencilCfg* best = !full && few_cells(g, d) ? default_segments(c, g, d, elem, 2, 128, 2.0) : nullptr;
     if (!best && elem == 8) {
         std::vector<PencilCfg> two;
         for (const PencilCfg& p : c)
@@ -1468,7 +1470,7 @@ int img_create(img_ctx** out, const img_config* cfg) {
         for (int d = 0; d < 3; ++d) {
             ctx->pcfg[kind][d] = choose_pencil(g, d, ctx->elem);
             if (kind == 0) {
-                ctx->pcfg_tile[d] = ctx->pcfg[0][d];
+                ctx->pcfg_tile[d] = ctx->pcfg_full[d] = ctx->pcfg[0][d];
                 if (tile_only) continue;
                 ctx->pcfg[0][d] = choose_fluid(g, d, ctx->elem, ctx->pcfg_tile[d], false);
             } else {
@@ -1492,8 +1494,10 @@ int img_create(img_ctx** out, const img_config* cfg) {
             if (it != g_tuned.end()) ctx->pcfg[kind][d] = it->second;
             if (kind == 0) {
                 ctx->pcfg_full[d] = ctx->pcfg[0][d];
-                const PencilCfg f = choose_fluid(g, d, ctx->elem, ctx->pcfg_tile[d], true);
-                if (it == g_tuned.end() && !tile_only && f.seg) ctx->pcfg_full[d] = f;   // (the same kernel family)
+                if (it == g_tuned.end() && ctx->pcfg[0][d].seg && few_cells(g, d)) {
+                    const PencilCfg f = choose_fluid(g, d, ctx->elem, ctx->pcfg_tile[d], true);
+                    if (f.seg) ctx->pcfg_full[d] = f;   // (the same kernel family)
+                }
             }
         }
 

@@ -37,3 +37,25 @@ def test_grids_of_many_sizes_share_launches(bc, magnet, dims, precision):
     b.close()
     for r in runs + alone:
         r.close()
+
+
+def test_members_on_the_tile_kernels_equal_their_runs_alone(monkeypatch):
+    """Contexts created with IMOGEN_B200_TILE_KERNELS=1 keep the tile kernels in a batch that fills the chip."""
+    monkeypatch.setenv("IMOGEN_B200_TILE_KERNELS", "1")
+    runs, alone = [], []
+    for i, n in enumerate((200, 150, 260, 90, 230)):
+        for lst in (runs, alone):
+            r = ImogenRun(precision="mixed", grid=(n, n + i, 1), dgrid=(1 / 64,) * 3, gamma=5 / 3, cfl=0.35, bc="circ", limiter="vanleer",
+                          magnet=True, time_max=1e5, iter_max=10 ** 6)
+            assert not any(t[6] for t in r.tiling("fluid").values())
+            r.set_state(*smooth_state((n, n + i, 1), seed=i, mhd=True))
+            lst.append(r)
+    b = ImogenBatch(runs)
+    b.run(9)
+    for x, y in zip(runs, alone):
+        y.run(9)
+        sx, sy = x.state(), y.state()
+        assert all((sx[k] == sy[k]).all() for k in sx), x.grid
+    b.close()
+    for r in runs + alone:
+        r.close()
