@@ -328,7 +328,8 @@ int img_autotune(img_ctx* ctx, int trials);
  * first) or the window magnet kernels (circ or const) -- and 0 for the pencil-tile kernels}. */
 int img_get_tiling(const img_ctx* ctx, int dim, int out[7]);
 /* Set the tiling of slot dim to one of those the autotuner may pick (same field order); a magnet
- * slot sets the chain's and the CT pass's tiling. */
+ * slot sets the chain's and the CT pass's tiling.  In the mixed form a segment tiling of the fluid sweep that is
+ * picked here or by img_autotune may round the last bits otherwise than the default tiling does. */
 int img_set_tiling(img_ctx* ctx, int dim, const int cfg[7]);
 
 /* Number of kernels the context has launched so far.  No reference counterpart. */
