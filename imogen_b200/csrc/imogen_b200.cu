@@ -558,9 +558,9 @@ const PencilCfg* default_segments(const std::vector<PencilCfg>& c, const Geom& g
 }
 
 // Grids whose threads of 4 cells would not fill the chip (under 148 x 256 of them): there each thread's own chain
-// of work is what takes the time, and 2 cells a thread in CTAs of 128 make the faster fluid sweeps (one iteration: 64^2
-// mixed 53 -> 45 us, 64^2 FP64 89 -> 75 us, 24^3 mixed 78 -> 68 us; 200^2 60 -> 57 us; 512^2 is past the line: x fluid
-// sweep 7.5 us with 4 cells, 9.2 us with 2).
+// of work is what takes the time, and 2 cells a thread in CTAs of 128 make the faster fluid sweeps (one iteration, 4 and
+// 2 cells: 64^2 mixed 53 and 46 us, FP64 99 and 82; 200^2 mixed 65 and 62, FP64 107 and 97; 512^2 is past the line:
+// mixed 100 and 130, FP64 174 and 187).
 constexpr long long kFullCells = 4 * 148 * 256;
 bool small_grid(const Geom& g) { return g.ncell < kFullCells; }
 
@@ -569,7 +569,7 @@ bool few_cells(const Geom& g, int d) { return small_grid(g) && g.n[d] <= 256; }
 
 // Default magnet tiling: the window kernels where a default window tiling exists, else the tile kernels'
 // default.  4 cells a thread and CTAs of 256 threads (512 share an SM by two as well: rows of 32 bytes come
-// first; 256^3 mixed, y: 8 pencils in 512 threads 355 us, 4 in 256 threads 476 us).
+// first; 256^3 mixed, y: 8 pencils in 512 threads 355 us, 4 in 256 threads 461 us).
 PencilCfg choose_window(const Geom& g, int d, size_t elem, const PencilCfg& tile) {
     std::vector<PencilCfg> c = win_candidates(g, d);
     const PencilCfg* best = default_segments(c, g, d, elem, 4, small_grid(g) ? 128 : 256, 1.0);
@@ -578,8 +578,8 @@ PencilCfg choose_window(const Geom& g, int d, size_t elem, const PencilCfg& tile
 
 // Default fluid tiling: the segment kernel where a default segment tiling exists, else the tile kernels'
 // default.  Mixed: 4 cells a thread, CTAs of 128 threads along x and 256 along y and z; one of 512 has an SM to
-// itself and nothing to hide its barriers behind (256^3, an earlier build: x 324 us with 64 to 128 threads, 355 with
-// 256, 425 with 512; y 504 us with 4 pencils in 256 threads, 534 with 8 in 512).  FP64: 2 cells a thread while two CTAs'
+// itself and nothing to hide its barriers behind (256^3: x 342 us with 64 to 128 threads, 376 with 256, 453 with
+// 512; y 526 us with 4 pencils in 256 threads, 568 with 8 in 512).  FP64: 2 cells a thread while two CTAs'
 // exchange records fit an SM (192 threads; 96^3 x 57 us, y 66 us), else 4 (96^3: 71 and 74 us; 128^3 y: 152 us,
 // with 2 cells in 256 threads 235 us).
 // `full`: beside other grids of a batch that fill the chip together.
